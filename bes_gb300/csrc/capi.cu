@@ -8,7 +8,7 @@
 #include <new>
 
 #include "context.hpp"
-#include "explicit_kernels.cuh"
+#include "side_kernels.cuh"
 
 using namespace bes;
 
@@ -67,14 +67,13 @@ int check_nan(bes_ctx* ctx) {
   return BES_OK;
 }
 
-// Enqueue one explicit multi-step iteration on ctx->stream (SolverExplicit::timeStep_), with
-// an event pair around every kernel so per-kernel device times of the last iteration can be
-// read back (bes_last_kernel_times).
+// Enqueue one explicit multi-step iteration on ctx->stream (SolverExplicit::timeStep_).  Every
+// kernel stores its start time, from which bes_last_kernel_times is read back (event-record
+// nodes around the kernels doubled the time of an iteration on a small mesh).
 void enqueue_iteration(bes_ctx* ctx, int cur) {
   const bes_options& o = ctx->opt;
   const DevMesh& m = ctx->dm;
-  const int nb_c = blocks_for(m.nc), nb_f = blocks_for(m.nf);
-  const dim3 gc(nb_c, ctx->nb), gf(nb_f, ctx->nb);  // y: condition
+  const dim3 gu((unsigned)((m.nc + kUpdBlock - 1) / kUpdBlock), ctx->nb);  // y: condition
   double* Un = ctx->U[cur];
   double* Uk = ctx->U[cur ^ 1];
   const int local = o.local_time_step;
@@ -82,40 +81,24 @@ void enqueue_iteration(bes_ctx* ctx, int cur) {
   freestream_step_kernel<<<1, 128, 0, s>>>(ctx->prm, ctx->nb, ctx->step_dev, ctx->pinf_dev,
                                            ctx->dtmin, ctx->iter_ctr, ctx->iter_cur);
   for (int k = 0; k < o.n_stage; ++k) {
-    cudaEvent_t* e = ctx->kev[k];
+    unsigned long long* st = ctx->stamps + 3 * k;
     const double* Uin = (k == 0) ? Un : Uk;
-    cudaEventRecordWithFlags(e[0], s, cudaEventRecordExternal);
-    if (k == 0)
-      cell_recon_kernel<true, false><<<gc, kBlock, 0, s>>>(
-          m, ctx->prm, Uin, ctx->RS, ctx->rs_ld, ctx->dt, o.courant_num, local, ctx->dtmin,
-          nullptr, nullptr);
-    else
-      cell_recon_kernel<false, false><<<gc, kBlock, 0, s>>>(
-          m, ctx->prm, Uin, ctx->RS, ctx->rs_ld, ctx->dt, o.courant_num, local, ctx->dtmin,
-          nullptr, nullptr);
-    cudaEventRecordWithFlags(e[1], s, cudaEventRecordExternal);
-    cudaEventRecordWithFlags(e[2], s, cudaEventRecordExternal);
-    face_flux_kernel<false><<<gf, kBlock, 0, s>>>(m, ctx->prm, ctx->RS, ctx->rs_ld, ctx->FA,
-                                                  nullptr, ctx->nan_flag);
-    cudaEventRecordWithFlags(e[3], s, cudaEventRecordExternal);
-    cudaEventRecordWithFlags(e[4], s, cudaEventRecordExternal);
+    launch_side_residual(ctx, s, Uin, k == 0, o.courant_num, ctx->prm, st);
     if (k == o.n_stage - 1)
-      update_kernel<true><<<gc, kBlock, 0, s>>>(m, ctx->FA, Un, Uk, ctx->dt, ctx->dtmin, local,
-                                                o.stage_coeff[k], ctx->partials, nullptr,
-                                                ctx->prm.active);
+      update_kernel<true><<<dim3(ctx->upd_blocks, ctx->nb), kUpdBlock, 0, s>>>(
+          m, ctx->FA, Un, Uk, ctx->dt, ctx->dtmin, local, o.stage_coeff[k], ctx->partials, nullptr,
+          ctx->prm.active, st + 2);
     else
-      update_kernel<false><<<gc, kBlock, 0, s>>>(m, ctx->FA, Un, Uk, ctx->dt, ctx->dtmin, local,
-                                                 o.stage_coeff[k], ctx->partials, nullptr,
-                                                 ctx->prm.active);
-    cudaEventRecordWithFlags(e[5], s, cudaEventRecordExternal);
+      update_kernel<false><<<gu, kUpdBlock, 0, s>>>(m, ctx->FA, Un, Uk, ctx->dt, ctx->dtmin, local,
+                                                    o.stage_coeff[k], ctx->partials, nullptr,
+                                                    ctx->prm.active, st + 2);
   }
-  finalize_norms_kernel<<<ctx->nb, kBlock, 0, s>>>(ctx->partials, nb_c, ctx->hist, ctx->hist_cap,
-                                                   ctx->iter_cur);
+  finalize_norms_kernel<<<ctx->nb, 320, 0, s>>>(ctx->partials, ctx->upd_blocks, ctx->hist,
+                                                ctx->hist_cap, ctx->iter_cur,
+                                                ctx->stamps + 3 * o.n_stage);
 }
 
 int build_graphs(bes_ctx* ctx) {
-  for (int k = 0; k < 8; ++k)
-    for (int q = 0; q < 6; ++q) BES_CUDA_TRY(ctx, cudaEventCreate(&ctx->kev[k][q]));
   for (int cur = 0; cur < 2; ++cur) {
     cudaGraph_t g;
     BES_CUDA_TRY(ctx, cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
@@ -243,14 +226,19 @@ int create_context(const bes_mesh_arrays* mesh, const bes_options* opt, int n_co
   rc |= upload(c, &m.farea, S.farea);
   if (rc) return BES_ERR_CUDA;
   const int64_t nc = S.nc, nf = S.nf, nb = n_cond;
+  c->side_path = opt->solver_type != 1;
   c->rs_ld = nc * S.nslots + S.n_extra;
   rc |= dev_alloc(c, &c->U[0], 5 * nc * nb);
   rc |= dev_alloc(c, &c->U[1], 5 * nc * nb);
-  rc |= dev_alloc(c, &c->RS, 5 * c->rs_ld * nb);
-  rc |= dev_alloc(c, &c->FA, 5 * nf * nb);
+  rc |= dev_alloc(c, &c->RS, (c->side_path ? kSideW : 5) * c->rs_ld * nb);
+  rc |= dev_alloc(c, &c->FA, kFaW * nf * nb);
   rc |= dev_alloc(c, &c->dt, nc * nb);
-  c->max_blocks = blocks_for(nc);
-  rc |= dev_alloc(c, &c->partials, 10 * (size_t)c->max_blocks * nb);
+  c->upd_blocks = (int)std::min<int64_t>((nc + kUpdBlock - 1) / kUpdBlock, kUpdBlocks);
+  rc |= dev_alloc(c, &c->partials, 10 * (size_t)c->upd_blocks * nb);
+  rc |= dev_alloc(c, &c->stamps, 3 * 8 + 1);
+  double2* hmat = nullptr;
+  if (c->side_path) rc |= dev_alloc(c, &hmat, 8 * nc);
+  m.hmat = hmat;
   rc |= dev_alloc(c, &c->dtmin, nb);
   c->hist_cap = std::max<int64_t>(16, 4096 / nb);  // iterations per history chunk
   rc |= dev_alloc(c, &c->hist, 10 * c->hist_cap * nb);
@@ -270,10 +258,16 @@ int create_context(const bes_mesh_arrays* mesh, const bes_options* opt, int n_co
     BES_CUDA_TRY(c, cudaMemcpy(c->new2ref_dev, n2r.data(), nc * sizeof(int32_t),
                                cudaMemcpyHostToDevice));
   }
+  if (c->side_path)
+    face_matrix_kernel<<<(unsigned)((nc + 127) / 128), 128, 0, c->stream>>>(m, hmat);
+  BES_CUDA_TRY(c, cudaGetLastError());
   BES_CUDA_TRY(c, cudaMemset(c->iter_ctr, 0, sizeof(int64_t)));
   BES_CUDA_TRY(c, cudaMemset(c->nan_flag, 0, sizeof(int)));
   // gas and freestream (Config::initializePostMesh, src/Config.cpp:480-488), per condition
   c->prm.gas = make_gas(opt->gas_constant, opt->specific_heat_ratio, opt->harten_correction_limit);
+  c->prm.half_gm1 = 0.5 * c->prm.gas.gm1;
+  c->prm.two_gamma = 2.0 * c->prm.gas.gamma;
+  c->prm.gamma2_gm1 = c->prm.gas.gamma * c->prm.gas.gamma * c->prm.gas.gm1;
   c->pinf0_host.assign(6 * nb, 0.0);
   const int S_dim = c->ref.dim;
   for (int64_t b = 0; b < nb; ++b) {
@@ -295,12 +289,8 @@ int create_context(const bes_mesh_arrays* mesh, const bes_options* opt, int n_co
   c->prm.active = nb > 1 ? c->active_dev : nullptr;
   c->prm.ramp_steps = opt->freestream_ramp;
   c->prm.ramp_frac = opt->freestream_ramp_start_frac;
-  rc = build_graphs(c);
+  rc = opt->solver_type == 1 ? implicit_allocate(c) : build_graphs(c);
   if (rc) return rc;
-  if (opt->solver_type == 1) {
-    rc = implicit_allocate(c);
-    if (rc) return rc;
-  }
   rc = bes_set_freestream_state(c);
   if (rc) return rc;
   *out = ctx.release();
@@ -316,9 +306,6 @@ void bes_destroy(bes_ctx* ctx) {
   if (ctx->stream) cudaStreamSynchronize(ctx->stream);
   for (int i = 0; i < 2; ++i)
     if (ctx->it_graph[i]) cudaGraphExecDestroy(ctx->it_graph[i]);
-  for (int k = 0; k < 8; ++k)
-    for (int q = 0; q < 6; ++q)
-      if (ctx->kev[k][q]) cudaEventDestroy(ctx->kev[k][q]);
   implicit_release(ctx);
   for (void* p : ctx->allocations) cudaFree(p);
   if (ctx->stream) cudaStreamDestroy(ctx->stream);
@@ -442,12 +429,21 @@ int bes_compute_operators(bes_ctx* ctx, double cfl, double* dt, double* grad, do
   freestream_at(c->prm, c->host_step, P);
   BES_CUDA_TRY(c, cudaMemcpyAsync(c->pinf_dev, P, sizeof(P), cudaMemcpyHostToDevice, c->stream));
   reset_dtmin_kernel<<<1, 1, 0, c->stream>>>(c->dtmin);
-  cell_recon_kernel<true, true><<<blocks_for(nc), kBlock, 0, c->stream>>>(
+  const int nb_u = (int)((nc + kUpdBlock - 1) / kUpdBlock);
+  auto residual_sum = [&] {
+    update_kernel<false><<<nb_u, kUpdBlock, 0, c->stream>>>(m, c->FA, Ucur, scratch, c->dt, c->dtmin,
+                                                            1, 0.0, c->partials, c->R, nullptr, nullptr);
+  };
+  if (c->side_path) {
+    // the residual of the explicit iteration, bit for bit
+    launch_side_residual(c, c->stream, Ucur, true, cfl, c->prm, nullptr);
+    residual_sum();
+  }
+  cell_recon_kernel<true><<<blocks_for(nc), kBlock, 0, c->stream>>>(
       m, c->prm, Ucur, c->RS, c->rs_ld, c->dt, cfl, 1, c->dtmin, c->G, c->PHI);
   face_flux_kernel<true><<<blocks_for(nf), kBlock, 0, c->stream>>>(m, c->prm, c->RS, c->rs_ld,
                                                                    c->FA, c->Fface, c->nan_flag);
-  update_kernel<false><<<blocks_for(nc), kBlock, 0, c->stream>>>(
-      m, c->FA, Ucur, scratch, c->dt, c->dtmin, 1, 0.0, c->partials, c->R);
+  if (!c->side_path) residual_sum();
   BES_CUDA_TRY(c, cudaGetLastError());
   BES_CUDA_TRY(c, cudaStreamSynchronize(c->stream));
   auto fetch = [&](const double* d, int64_t count) {
@@ -521,13 +517,16 @@ void* bes_stream(bes_ctx* ctx) { return ctx ? (void*)ctx->stream : nullptr; }
 int bes_last_kernel_times(bes_ctx* ctx, double* ms_out) {
   if (!ctx || !ms_out) return BES_ERR_INVALID;
   BES_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
+  if (ctx->iterations_done == 0) {
+    ctx->last_error = "no explicit iteration has run";
+    return BES_ERR_CUDA;
+  }
+  unsigned long long t[3 * 8 + 1];
+  BES_CUDA_TRY(ctx, cudaMemcpy(t, ctx->stamps, (3 * ctx->opt.n_stage + 1) * sizeof(t[0]),
+                               cudaMemcpyDeviceToHost));
   double acc[3] = {0, 0, 0};
   for (int k = 0; k < ctx->opt.n_stage; ++k)
-    for (int q = 0; q < 3; ++q) {
-      float ms = 0;
-      BES_CUDA_TRY(ctx, cudaEventElapsedTime(&ms, ctx->kev[k][2 * q], ctx->kev[k][2 * q + 1]));
-      acc[q] += ms;
-    }
+    for (int q = 0; q < 3; ++q) acc[q] += 1e-6 * (double)(t[3 * k + q + 1] - t[3 * k + q]);
   ms_out[0] = acc[0];
   ms_out[1] = acc[1];
   ms_out[2] = acc[2];

@@ -23,6 +23,7 @@ struct DevMesh {
   const uint8_t* extra_m;
   const int32_t *fown, *fnb, *fsrc_own, *fsrc_nb;
   const double *fn, *farea;
+  const double2* hmat;  // per cell the 4x4 face matrix of side_kernels.cuh (explicit contexts), or null
 };
 
 struct Params {
@@ -34,6 +35,7 @@ struct Params {
   const int32_t* active = nullptr;    // per condition: 0 = frozen (its state is kept)
   int32_t ramp_steps;      // FREESTREAM_RAMP
   double ramp_frac;        // FREESTREAM_RAMP_START_FRAC
+  double half_gm1, two_gamma, gamma2_gm1;  // (gamma-1)/2, 2 gamma, gamma^2 (gamma-1)
 };
 
 // Freestream primitives of step t (Config::getFreestreamPrimitiveVariables,
@@ -219,17 +221,19 @@ struct bes_ctx {
   // state: two snapshots (the reference's ping-pong, src/Solution.cpp:63-71)
   double* U[2] = {nullptr, nullptr};
   int cur = 0;  // snapshot holding the current state
-  double* RS = nullptr;  // reconstructed face-side states [5][rs_ld]
+  // explicit contexts run the kernels of side_kernels.cuh
+  bool side_path = false;
+  double* RS = nullptr;  // reconstructed face-side states [5][rs_ld], or side states [rs_ld][8]
   int64_t rs_ld = 0;
-  double* FA = nullptr;  // face flux x area [5][nf]
+  double* FA = nullptr;  // face flux x area [nf][6]
   double* dt = nullptr;  // [nc]
   double* G = nullptr;   // optional gradient output [15][nc]
   double* PHI = nullptr; // optional limiter output [5][nc]
   double* Fface = nullptr;  // optional flux per unit area [5][nf]
   double* R = nullptr;   // optional residual [5][nc]
   // reductions
-  double* partials = nullptr;  // [10][max_blocks]
-  int max_blocks = 0;
+  double* partials = nullptr;  // [10][upd_blocks]
+  int upd_blocks = 0;          // grid of the last stage's update
   unsigned long long* dtmin = nullptr;  // global time step as ordered bits
   double* hist = nullptr;               // device history [hist_cap][10]
   int64_t hist_cap = 0;
@@ -252,9 +256,9 @@ struct bes_ctx {
   int64_t host_step = 0;          // the same counter on the host
   // graphs: one explicit iteration for each parity of the current snapshot
   cudaGraphExec_t it_graph[2] = {nullptr, nullptr};
-  // event pairs around every kernel of an explicit iteration (graph event-record nodes):
-  // [stage][0/1 cell, 2/3 face, 4/5 update]
-  cudaEvent_t kev[8][6] = {};
+  // start times of the kernels of the last explicit iteration, [stage][cell, face, update],
+  // then the norms kernel's
+  unsigned long long* stamps = nullptr;
   int64_t iterations_done = 0;
   int64_t iters_since_reset = 0;  // graph launches since the history counter was reset
   bes::ImplicitBuffers imp;

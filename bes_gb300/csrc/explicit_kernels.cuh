@@ -1,18 +1,49 @@
-// Kernels of the explicit residual/update path (FP64).  One explicit stage is three sweeps:
+// Kernels of the residual/update path (FP64).  A residual is three sweeps:
 //   cell_recon_kernel  per cell: Green-Gauss gradient (GradientGreenGauss.cpp:21-135),
 //                      Venkatakrishnan limiter (LimiterVenkatakrishnan.cpp:21-128) and the
-//                      MUSCL face-side states (Solver.cpp:69-121), fused; at stage 0 also the
-//                      local time step (TimeStepCalculatorLocal.cpp:67-93).
+//                      MUSCL face-side states (Solver.cpp:69-121), fused, with the local time
+//                      step (TimeStepCalculatorLocal.cpp:67-93).
 //   face_flux_kernel   per face: Roe / slip-wall / freestream flux times area.
 //   update_kernel      per cell: R = sum of +-flux*area in the reference's face order, then
 //                      W(k) = W(n) - alpha_k dt/V R (SolverExplicit.cpp:326-378); the last stage
 //                      also reduces the L2 / max norms of R.
+// The first two serve the operator entry points (which return gradient, limiter and face
+// states) and the implicit steps; explicit iterations run their counterparts of
+// side_kernels.cuh.
 #pragma once
 #include "context.hpp"
 
 namespace bes {
 
 constexpr int kBlock = 256;
+// Face fluxes times area are face-major, FA [nf][kFaW] (five values and a pad): a cell reads a
+// face's five values as three 16-byte loads of one or two sectors instead of five loads of
+// five sectors.
+constexpr int kFaW = 6;
+
+// Start time of a kernel (the GPU's nanosecond timer) for bes_last_kernel_times.
+__device__ __forceinline__ void stamp_start(unsigned long long* stamp) {
+  if (stamp != nullptr && threadIdx.x == 0 && blockIdx.x == 0 && blockIdx.y == 0) {
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+    *stamp = t;
+  }
+}
+__device__ __forceinline__ void store_fa(double* __restrict__ FA, int f, const double* F) {
+  double2* o = reinterpret_cast<double2*>(FA + (int64_t)f * kFaW);
+  o[0] = make_double2(F[0], F[1]);
+  o[1] = make_double2(F[2], F[3]);
+  o[2] = make_double2(F[4], 0.0);
+}
+__device__ __forceinline__ void load_fa(const double* __restrict__ FA, int f, double* F) {
+  const double2* o = reinterpret_cast<const double2*>(FA + (int64_t)f * kFaW);
+  const double2 a = o[0], b = o[1];
+  F[0] = a.x;
+  F[1] = a.y;
+  F[2] = b.x;
+  F[3] = b.y;
+  F[4] = FA[(int64_t)f * kFaW + 4];
+}
 
 __device__ __forceinline__ double warp_sum(double x) {
 #pragma unroll
@@ -40,7 +71,7 @@ __device__ __forceinline__ bool condition_frozen(const Params& prm) {
 
 // Cell sweep.  U is [5][nc]; RS is [5][ldr] with ldr >= nc*nslots + n_extra.  cfl_dev (may
 // be null): a per-condition CFL number that replaces cfl (the implicit step's CFL control).
-template <bool STAGE0, bool WRITE_GL>
+template <bool WRITE_GL>
 __global__ void __launch_bounds__(kBlock) cell_recon_kernel(
     DevMesh m, Params prm, const double* __restrict__ U, double* __restrict__ RS, int64_t ldr,
     double* __restrict__ dt, double cfl, int local_dt, unsigned long long* __restrict__ dtmin,
@@ -183,7 +214,7 @@ __global__ void __launch_bounds__(kBlock) cell_recon_kernel(
         for (int d = 0; d < 3; ++d) G_out[(int64_t)(v * 3 + d) * nc + c] = G[v][d];
       }
     }
-    if (STAGE0) {
+    {
       // local time step: CFL V / sum_d (c~ + |u_d|) L_d with c~ = sqrt(gamma) c (quirk Q3)
       const double ir = 1.0 / u[0];
       const double k2 = u[1] * u[1] + u[2] * u[2] + u[3] * u[3];
@@ -199,13 +230,13 @@ __global__ void __launch_bounds__(kBlock) cell_recon_kernel(
       dt[c] = dt_c;
     }
   }
-  if (STAGE0 && !local_dt) {
+  if (!local_dt) {
     __shared__ double smin[kBlock / 32];
     double x = warp_min(dt_c);
     if ((threadIdx.x & 31) == 0) smin[threadIdx.x >> 5] = x;
     __syncthreads();
     if (threadIdx.x < 32) {
-      x = threadIdx.x < kBlock / 32 ? smin[threadIdx.x] : 1e300;
+      x = threadIdx.x < blockDim.x / 32 ? smin[threadIdx.x] : 1e300;
       x = warp_min(x);
       // positive doubles order like their bit patterns
       if (threadIdx.x == 0) atomicMin(dtmin, (unsigned long long)__double_as_longlong(x));
@@ -222,7 +253,7 @@ __global__ void __launch_bounds__(kBlock) face_flux_kernel(
   if (f >= nf || condition_frozen(prm)) return;
   const int64_t b = blockIdx.y;
   RS += b * 5 * ldr;
-  FA += b * 5 * nf;
+  FA += b * kFaW * nf;
   const double* pinf = prm.pinf_dev + 6 * b;
   double UL[5], F[5];
   const int so = m.fsrc_own[f];
@@ -246,24 +277,33 @@ __global__ void __launch_bounds__(kBlock) face_flux_kernel(
   bool bad = false;
 #pragma unroll
   for (int v = 0; v < 5; ++v) {
-    FA[(int64_t)v * nf + f] = F[v] * A;
     if (WRITE_F) F_out[(int64_t)v * nf + f] = F[v];
     bad |= (F[v] != F[v]);
+    F[v] *= A;
   }
+  store_fa(FA, f, F);
   if (bad) atomicCAS(nan_flag, 0, f + 1);
 }
 
+// Blocks of the last stage's update: at most eight per SM, each looping over the cells, so that
+// a thread adds up its cells' squares before the block reduction.
+constexpr int kUpdBlock = 128;
+constexpr int kUpdBlocks = 1216;
+
+// R and the stage update; bound by the gathers of the four faces' fluxes (L2).  LAST: also the
+// per-block partial norms of R, partials[k*gridDim.x + block].
 template <bool LAST>
-__global__ void __launch_bounds__(kBlock) update_kernel(
+__global__ void __launch_bounds__(kUpdBlock) update_kernel(
     DevMesh m, const double* __restrict__ FA, const double* __restrict__ Un,
     double* __restrict__ Uout, const double* __restrict__ dt,
     const unsigned long long* __restrict__ dtmin, int local_dt, double alpha,
-    double* __restrict__ partials, double* __restrict__ R_out, const int32_t* active = nullptr) {
+    double* __restrict__ partials, double* __restrict__ R_out, const int32_t* active,
+    unsigned long long* stamp) {
   const int nc = m.nc, nf = m.nf;
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  stamp_start(stamp);
   {
     const int64_t b = blockIdx.y;
-    FA += b * 5 * nf;
+    FA += b * kFaW * nf;
     Un += b * 5 * nc;
     Uout += b * 5 * nc;
     dt += b * nc;
@@ -272,22 +312,27 @@ __global__ void __launch_bounds__(kBlock) update_kernel(
   }
   const bool frozen = active != nullptr && active[blockIdx.y] == 0;
   if (frozen && !LAST) return;
-  double R[5] = {0, 0, 0, 0, 0};
-  if (frozen) {
-    // keep the state: the last stage's output becomes the next iteration's input
-    if (c < nc)
+  double sum[5] = {0, 0, 0, 0, 0};
+  long long top[5] = {0, 0, 0, 0, 0};  // bit patterns of max |R| (order like the values)
+  for (int c = blockIdx.x * kUpdBlock + threadIdx.x; c < nc; c += gridDim.x * kUpdBlock) {
+    if (frozen) {
+      // keep the state: the last stage's output becomes the next iteration's input
 #pragma unroll
       for (int v = 0; v < 5; ++v) Uout[(int64_t)v * nc + c] = Un[(int64_t)v * nc + c];
-  } else if (c < nc) {
+      continue;
+    }
+    double R[5] = {0, 0, 0, 0, 0};
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
       const int g = m.gface[q * nc + c];
       if (g == bes::kNoFace) continue;  // empty slot of a triangle
-      const int f = g >= 0 ? g : ~g;
+      double F[5];
+      load_fa(FA, g >= 0 ? g : ~g, F);
+      const long long flip = g >= 0 ? 0ll : (long long)0x8000000000000000ull;
 #pragma unroll
       for (int v = 0; v < 5; ++v) {
-        const double x = FA[(int64_t)v * nf + f];
-        R[v] = g >= 0 ? R[v] + x : R[v] - x;
+        const double x = __longlong_as_double(__double_as_longlong(F[v]) ^ flip);
+        R[v] = q == 0 ? x : R[v] + x;
       }
     }
     const double dtc = local_dt ? dt[c] : __longlong_as_double((long long)*dtmin);
@@ -297,57 +342,66 @@ __global__ void __launch_bounds__(kBlock) update_kernel(
     if (R_out)
 #pragma unroll
       for (int v = 0; v < 5; ++v) R_out[(int64_t)v * nc + c] = R[v];
+    if (LAST)
+#pragma unroll
+      for (int v = 0; v < 5; ++v) {
+        sum[v] = fma(R[v], R[v], sum[v]);
+        const long long a = __double_as_longlong(R[v]) & 0x7fffffffffffffffll;
+        if (a > top[v] && a <= 0x7ff0000000000000ll) top[v] = a;  // a NaN is no maximum
+      }
+    if (!LAST) break;
   }
   if (LAST) {
-    __shared__ double sh[10][kBlock / 32];
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    // through shared memory: 16 threads per row add eight values each, then four shuffle
+    // levels, so that few warps spend FP64 additions on it
+    __shared__ double sh[5][kUpdBlock + 4];
+    __shared__ long long st[5][kUpdBlock];
 #pragma unroll
     for (int v = 0; v < 5; ++v) {
-      const double s = warp_sum(R[v] * R[v]);
-      const double mx = warp_max(fabs(R[v]));
-      if (lane == 0) {
-        sh[v][wid] = s;
-        sh[5 + v][wid] = mx;
-      }
+      sh[v][threadIdx.x] = sum[v];
+      st[v][threadIdx.x] = top[v];
     }
     __syncthreads();
-    if (threadIdx.x < 32) {
+    const int row = threadIdx.x >> 4, part = threadIdx.x & 15;
+    double s = 0.0;
+    long long t = 0;
+    if (row < 5)
 #pragma unroll
-      for (int k = 0; k < 10; ++k) {
-        double x = lane < kBlock / 32 ? sh[k][lane] : 0.0;
-        x = k < 5 ? warp_sum(x) : warp_max(x);
-        if (lane == 0) partials[(int64_t)k * gridDim.x + blockIdx.x] = x;
+      for (int q = 0; q < kUpdBlock / 16; ++q) {
+        s += sh[row][q * 16 + part];
+        const long long x = st[row][q * 16 + part];
+        t = x > t ? x : t;
       }
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) {
+      s += __shfl_xor_sync(0xffffffffu, s, o);
+      const long long x = __shfl_xor_sync(0xffffffffu, t, o);
+      t = x > t ? x : t;
+    }
+    if (row < 5 && part == 0) {
+      partials[(int64_t)row * gridDim.x + blockIdx.x] = s;
+      partials[(int64_t)(5 + row) * gridDim.x + blockIdx.x] = __longlong_as_double(t);
     }
   }
 }
 
-// One block per condition: reduce the per-block partials in a fixed order into
-// history[iter][condition] (L2, max); iter = *iter_cur (set by freestream_step_kernel).
-static __global__ void __launch_bounds__(kBlock) finalize_norms_kernel(
+// One block per condition, one warp per norm: reduce the per-block partials in a fixed order
+// into history[iter][condition] (L2, max); iter = *iter_cur (set by freestream_step_kernel).
+static __global__ void __launch_bounds__(320) finalize_norms_kernel(
     const double* __restrict__ partials, int nblocks, double* __restrict__ hist,
-    int64_t hist_cap, const int64_t* __restrict__ iter_cur) {
-  __shared__ double sh[kBlock / 32];
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    int64_t hist_cap, const int64_t* __restrict__ iter_cur, unsigned long long* stamp) {
+  stamp_start(stamp);
+  const int lane = threadIdx.x & 31, k = threadIdx.x >> 5;
   const int64_t it = *iter_cur;
   const int nb = gridDim.x, b = blockIdx.x;
-  partials += (int64_t)b * 10 * nblocks;
-  for (int k = 0; k < 10; ++k) {
-    double x = 0.0;
-    for (int b = threadIdx.x; b < nblocks; b += blockDim.x) {
-      const double y = partials[(int64_t)k * nblocks + b];
-      x = k < 5 ? x + y : fmax(x, y);
-    }
-    x = k < 5 ? warp_sum(x) : warp_max(x);
-    if (lane == 0) sh[wid] = x;
-    __syncthreads();
-    if (threadIdx.x < 32) {
-      x = lane < kBlock / 32 ? sh[lane] : 0.0;
-      x = k < 5 ? warp_sum(x) : warp_max(x);
-      if (lane == 0 && it < hist_cap) hist[(it * nb + b) * 10 + k] = k < 5 ? sqrt(x) : x;
-    }
-    __syncthreads();
+  const double* __restrict__ row = partials + ((int64_t)b * 10 + k) * nblocks;
+  double x = 0.0;
+  for (int q = lane; q < nblocks; q += 32) {
+    const double y = row[q];
+    x = k < 5 ? x + y : fmax(x, y);
   }
+  x = k < 5 ? warp_sum(x) : warp_max(x);
+  if (lane == 0 && it < hist_cap) hist[(it * nb + b) * 10 + k] = k < 5 ? sqrt(x) : x;
 }
 
 static __global__ void reset_dtmin_kernel(unsigned long long* dtmin) {

@@ -39,6 +39,11 @@ namespace {
 
 inline int nblk(int64_t n, int b) { return (int)((n + b - 1) / b); }
 
+// Threads of a block of the residual kernels: one warp while every warp can have an SM
+// sub-partition almost to itself (152 SMs x 4 x 32 threads, twice), because they are chains of
+// FP64 instructions that take 64 cycles each (1,152 cells: cell sweep 50 us in 5 blocks of 256).
+inline int residual_block(int64_t n) { return n <= 38912 ? 32 : kBlock; }
+
 int imp_malloc(bes_ctx* c, void** p, size_t bytes) {
   cudaError_t e = cudaMalloc(p, bytes ? bytes : 8);
   if (e != cudaSuccess) {
@@ -464,10 +469,11 @@ void enqueue_residual_all(bes_ctx* c, cudaStream_t s, const SlotHandles& hs, int
   Params prm = c->prm;
   prm.active = c->imp.act;
   stamp(c, s, PROF_RESIDUAL, 1);
-  cell_recon_kernel<true, false><<<dim3(nblk(m.nc, kBlock), nslot), kBlock, 0, s>>>(
+  const int bc = residual_block((int64_t)m.nc * nslot), bf = residual_block((int64_t)m.nf * nslot);
+  cell_recon_kernel<false><<<dim3(nblk(m.nc, bc), nslot), bc, 0, s>>>(
       m, prm, c->U[c->cur], c->RS, c->rs_ld, c->dt, 0.0, c->opt.local_time_step, c->dtmin,
       nullptr, nullptr, c->imp.cfl_dev);
-  face_flux_kernel<false><<<dim3(nblk(m.nf, kBlock), nslot), kBlock, 0, s>>>(
+  face_flux_kernel<false><<<dim3(nblk(m.nf, bf), nslot), bf, 0, s>>>(
       m, prm, c->RS, c->rs_ld, c->FA, nullptr, c->nan_flag);
   stamp(c, s, PROF_RESIDUAL, 0);
 }
@@ -505,7 +511,7 @@ void enqueue_assembly(const Sys<T, B>& S, cudaStream_t s, int k, double* norms) 
   stamp(c, s, PROF_JACOBIAN, 0);
   stamp(c, s, PROF_ASSEMBLE, 1);
   const int nb = nblk(nc, 128);
-  cell_assemble_kernel<T><<<nb, 128, 0, s>>>(m, c->FA + k * 5 * nf, dt, dtmin, local,
+  cell_assemble_kernel<T><<<nb, 128, 0, s>>>(m, c->FA + k * kFaW * nf, dt, dtmin, local,
                                              o.jacobian_repeat, S.Dc, A,
                                              uses_ilu(c) ? nullptr : Dinv,
                                              c->imp.rhs + k * 5 * nc, S.b + k * S.ldv, red);

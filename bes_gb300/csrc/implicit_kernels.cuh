@@ -194,12 +194,13 @@ __global__ void __launch_bounds__(128) cell_assemble_kernel(
       const int gf = m.gface[s * nc + i];
       if (gf == bes::kNoFace) continue;  // empty slot of a triangle
       const int f = gf >= 0 ? gf : ~gf;
+      double fa[5];
+      load_fa(FA, f, fa);
 #pragma unroll
       for (int v = 0; v < 5; ++v) {
-        const double fa = FA[(int64_t)v * nf + f];
-        const double x = k * fa;
+        const double x = k * fa[v];
         b[v] = gf >= 0 ? b[v] - x : b[v] + x;
-        R[v] = gf >= 0 ? R[v] + fa : R[v] - fa;
+        R[v] = gf >= 0 ? R[v] + fa[v] : R[v] - fa[v];
       }
       const T* src = Dc + (gf >= 0 ? 0 : (int64_t)25 * nf);
 #pragma unroll

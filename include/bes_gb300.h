@@ -211,7 +211,7 @@ int bes_flux_batch(bes_ctx* ctx, int32_t kind, int64_t n, const double* UL, cons
  * bes_synchronize waits and reports a NaN flux or CUDA error of the enqueued work;
  * bes_stream returns the context's cudaStream_t; bes_last_kernel_times gives the device
  * milliseconds of the most recent iteration's kernels (ms_out [4]: cell sweep, face flux,
- * update, sum), read from event pairs captured around every kernel. */
+ * update, sum), each from the kernel's start to the next kernel's start by the GPU's timer. */
 int bes_explicit_enqueue(bes_ctx* ctx, int64_t n);
 int bes_synchronize(bes_ctx* ctx);
 void* bes_stream(bes_ctx* ctx);
