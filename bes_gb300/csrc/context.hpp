@@ -170,6 +170,10 @@ struct ImplicitBuffers {
   int sweep_kernel = 1;        // 1 per colour, 2 persistent, 3 per colour with loads first
   bool tuned = false;
   int persistent_blocks = 0;   // grid of the persistent sweep
+  int solve_blocks = 0;        // grid of the persistent linear solve; 0: the step graph's solve
+  bool solve_lane_spmv = false;  // the row form of its products
+  void* Y = nullptr;           // its forward-solve vector [ldv], per condition
+  int solve_resident = 0;      // blocks of it that can be resident
   unsigned int* sync_count = nullptr;  // grid barrier: arrivals, generation, error flag
   unsigned int* sync_gen = nullptr;
   int* sync_error = nullptr;

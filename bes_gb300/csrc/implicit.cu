@@ -11,8 +11,8 @@
 // frozen slot), then the linear solves of all slots together: a WHILE node over restart
 // cycles whose body holds one IF node per Arnoldi step, the Arnoldi kernels batched over the
 // slots and the GMRES bookkeeping (Hessenberg column, Givens rotations, least squares,
-// restart and convergence) in small device kernels (krylov_kernels.cuh).  The host reads the
-// step's norms and linear-solve statistics back once per step and runs the CFL control.
+// restart and convergence) in small device kernels (krylov_kernels.cuh); or, on small meshes, one
+// persistent kernel (gmres_persistent.cuh).  The host reads the step's norms and linear-solve statistics back once per step and runs the CFL control.
 #include <algorithm>
 #include <cmath>
 #include <cstddef>
@@ -22,7 +22,7 @@
 #include <vector>
 
 #include "context.hpp"
-#include "krylov_kernels.cuh"
+#include "gmres_persistent.cuh"
 
 using namespace bes;
 
@@ -204,15 +204,9 @@ bool sweep_plan(const SoaMesh& M, SweepPlan& P) {
   return true;
 }
 
-// One persistent launch of the whole colour sweep from `in` into Z (cooperative: every block
-// of the grid is resident, which the grid barrier between colours needs).
+// Operands of the colour sweeps (or of block Jacobi: the inverse diagonal only).
 template <class T, class B>
-cudaError_t launch_persistent_sweep(const Sys<T, B>& S, cudaStream_t s, SlotPtr<const T> in,
-                                    const int32_t* run) {
-  bes_ctx* c = S.c;
-  const ImplicitBuffers& I = c->imp;
-  SweepPlan P;
-  if (!sweep_plan(c->soa, P)) return cudaErrorInvalidConfiguration;
+SweepOps<T> sweep_ops(const Sys<T, B>& S) {
   SweepOps<T> O;
   std::memset(&O, 0, sizeof(O));
   if (S.packed) {
@@ -224,6 +218,19 @@ cudaError_t launch_persistent_sweep(const Sys<T, B>& S, cudaStream_t s, SlotPtr<
     O.L = cslots((const T*)S.LU, S.sA);
     O.Dinv = cslots((const T*)S.Dinv, S.sDinv);
   }
+  return O;
+}
+
+// One persistent launch of the whole colour sweep from `in` into Z (cooperative: every block
+// of the grid is resident, which the grid barrier between colours needs).
+template <class T, class B>
+cudaError_t launch_persistent_sweep(const Sys<T, B>& S, cudaStream_t s, SlotPtr<const T> in,
+                                    const int32_t* run) {
+  bes_ctx* c = S.c;
+  const ImplicitBuffers& I = c->imp;
+  SweepPlan P;
+  if (!sweep_plan(c->soa, P)) return cudaErrorInvalidConfiguration;
+  SweepOps<T> O = sweep_ops(S);
   O.in = in;
   O.out = S.vec(S.Z);
   const GridSync gs{I.sync_count, I.sync_gen, I.sync_error};
@@ -243,6 +250,62 @@ cudaError_t launch_persistent_sweep(const Sys<T, B>& S, cudaStream_t s, SlotPtr<
                                 S.nslot, run, gs);
   return cudaLaunchKernelEx(&cfg, ilu_sweep_persistent_kernel<T, false>, c->dm, P, O, S.nslot,
                             run, gs);
+}
+
+// The linear solves of the step as one cooperative launch (gmres_persistent.cuh).
+template <class T, class B>
+int enqueue_persistent_solve(const Sys<T, B>& S, cudaStream_t s, const GmresParam& P, int prof) {
+  bes_ctx* c = S.c;
+  const ImplicitBuffers& I = c->imp;
+  SolveArgs<T, B> a;
+  std::memset(&a, 0, sizeof(a));
+  a.m = c->dm;
+  a.ilu = uses_ilu(c);
+  if (a.ilu && !sweep_plan(c->soa, a.plan)) return BES_ERR_UNSUPPORTED;
+  a.ops = sweep_ops(S);
+  if (S.packed) {
+    a.A16 = cslots((const __half2*)S.A16, 65LL * S.nc);
+    a.As = cslots((const float*)S.As, 5LL * S.nc);
+  } else {
+    a.A = cslots((const T*)S.A, S.sA);
+  }
+  a.b = S.cvec(S.b);
+  a.Y = S.vec((T*)I.Y);
+  a.Z = S.vec(S.Z);
+  a.W = S.vec(S.W);
+  a.X = S.vec(S.X);
+  a.Vx = S.vec(S.Vx);
+  a.V = S.V;
+  a.sV = S.sV;
+  a.ldv = S.ldv;
+  a.N = S.N;
+  a.red = I.red;
+  a.sred = 64 * I.red_ld;
+  a.g = I.gm;
+  a.P = P;
+  a.nslot = S.nslot;
+  a.lane_spmv = I.solve_lane_spmv;
+  a.act = I.act;
+  a.nan_flag = c->nan_flag;
+  a.guard = I.guard_dev;
+  a.bar = GridBar{I.sync_count, I.sync_error};
+  a.prof = prof ? c->prof.dev : nullptr;
+  IMP_TRY(c, cudaMemsetAsync(I.sync_count, 0, sizeof(unsigned), s));
+  cudaLaunchConfig_t cfg;
+  std::memset(&cfg, 0, sizeof(cfg));
+  cfg.gridDim = dim3(I.solve_blocks);
+  cfg.blockDim = dim3(256);
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeCooperative;
+  at[0].val.cooperative = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  if constexpr (std::is_same<T, float>::value && !std::is_same<T, B>::value)
+    IMP_TRY(c, cudaLaunchKernelEx(&cfg, gmres_solve_kernel<T, B, true>, a));
+  else
+    IMP_TRY(c, cudaLaunchKernelEx(&cfg, gmres_solve_kernel<T, B, false>, a));
+  return BES_OK;
 }
 
 // Z = M^{-1} in for every slot whose run flag is set
@@ -568,6 +631,33 @@ int reset_grid_sync(bes_ctx* c) {
   return BES_OK;
 }
 
+// The linear solves as one persistent launch (gmres_persistent.cuh) or as the graph's kernels:
+// persistent while the rows between two waits (a colour, or all of them with block Jacobi) are
+// no more than a few times what the grid's warps hold at six rows each.  A step's solve, graph
+// against persistent, measured (ms, one step at CFL 50): block ILU 7k cells FP32 4.5 / 2.2, 20k
+// FP64 9.0 / 4.8, 74k packed 7.8 / 5.9, FP32 10.5 / 6.6, FP64 20.5 / 14.9, 5 x 20k packed 8.2 / 6.3,
+// 150k FP32 23.5 / 15.1; 150k packed 11.5 / 14.5 (2.2 times: its sweeps are the fast ones of the
+// graph).  Block Jacobi: 20k FP64 12.2 / 8.6, 74k FP32 11.2 / 8.8 (5.1 times).
+void choose_solve(bes_ctx* c) {
+  ImplicitBuffers& I = c->imp;
+  I.solve_blocks = 0;
+  SweepPlan plan;
+  if (c->opt.sweep_kernel != 0 || c->opt.linear_solver == 2 || I.solve_resident < 1) return;
+  if (uses_ilu(c) && (!I.use_colour_ranges || !sweep_plan(c->soa, plan))) return;
+  const int64_t rows = (int64_t)c->soa.nc * I.nslot;
+  int64_t stage = rows;
+  if (uses_ilu(c)) {
+    stage = 0;
+    for (int q = 0; q < plan.n; ++q) stage = std::max(stage, (int64_t)(plan.r1[q] - plan.r0[q]) * I.nslot);
+  }
+  const int64_t blocks = std::min<int64_t>(I.solve_resident, (rows + 31) / 32);
+  const double held = (double)kRowsPerWarp * 8 * blocks;
+  if (stage > held * (!uses_ilu(c) ? 5.5 : (I.packed ? 1.75 : 2.5))) return;
+  I.solve_lane_spmv = rows <= 1.25 * held;
+  if (uses_ilu(c) && !I.Y && imp_malloc(c, &I.Y, I.ldv * I.tsize * I.nslot)) return;
+  I.solve_blocks = (int)blocks;
+}
+
 // The colour-sweep variant, timed on this context's mesh and slots: one launch per colour, or
 // one persistent launch per sweep.  Each candidate runs 3 untimed and 10 timed sweeps (CUDA
 // events on the context's stream, all slots); a persistent candidate whose launch fails or
@@ -578,6 +668,15 @@ int tune_sweep(bes_ctx* c) {
   Sys<T, B> S(c);
   I.tuned = true;
   char line[256];
+  choose_solve(c);
+  if (I.solve_blocks > 0) {
+    std::snprintf(line, sizeof(line),
+                  "colour sweep: one launch per colour not timed; taken: the linear solves in one "
+                  "persistent launch (%d blocks of 256; %d slots, %d cells)\n",
+                  I.solve_blocks, S.nslot, S.nc);
+    I.tuning += line;
+    return BES_OK;
+  }
   if (!uses_ilu(c) || !I.use_colour_ranges) {
     I.sweep_kernel = 1;
     return BES_OK;
@@ -686,6 +785,21 @@ void abandon_capture(bes_ctx* c) {
   cudaGetLastError();
 }
 
+// The state update and the end of the step's capture.
+template <class T, class B>
+int end_step(const Sys<T, B>& S, cudaStream_t s0, int prof, cudaGraph_t* out) {
+  bes_ctx* c = S.c;
+  ImplicitBuffers& I = c->imp;
+  stamp(c, s0, PROF_OTHER, 1);
+  state_update_kernel<T><<<S.vgrid, 256, 0, s0>>>(slots(c->U[c->cur], 5LL * S.nc), S.cvec(S.X),
+                                                  (int64_t)S.nc, c->nan_flag, I.act);
+  stamp(c, s0, PROF_OTHER, 0);
+  IMP_TRY(c, cudaGetLastError());
+  IMP_TRY(c, cudaStreamEndCapture(s0, out));
+  I.nodes_top[prof] = kernel_nodes(*out);
+  return BES_OK;
+}
+
 template <class T, class B>
 int capture_step(bes_ctx* c, int prof, cudaGraph_t* out) {
   Sys<T, B> S(c);
@@ -703,8 +817,10 @@ int capture_step(bes_ctx* c, int prof, cudaGraph_t* out) {
   GmresHandles gh;
   std::memset(&gh, 0, sizeof(gh));
   gh.on = 1;
-  IMP_TRY(c, cudaGraphConditionalHandleCreate(&gh.loop, g, 0, cudaGraphCondAssignDefault));
-  for (int j = 0; j < o.gmres_restart; ++j) {
+  // (a handle without a node makes the graph invalid)
+  if (I.solve_blocks == 0)
+    IMP_TRY(c, cudaGraphConditionalHandleCreate(&gh.loop, g, 0, cudaGraphCondAssignDefault));
+  for (int j = 0; I.solve_blocks == 0 && j < o.gmres_restart; ++j) {
     IMP_TRY(c, cudaGraphConditionalHandleCreate(&gh.arn[j], g, 0, cudaGraphCondAssignDefault));
     IMP_TRY(c, cudaGraphConditionalHandleCreate(&gh.gs2[j], g, 0, cudaGraphCondAssignDefault));
   }
@@ -717,6 +833,11 @@ int capture_step(bes_ctx* c, int prof, cudaGraph_t* out) {
     enqueue_factor(S, s1, k);
     if ((rc = end_conditional(c, s1, &I.nodes_slot[prof]))) return rc;
   }
+  if (I.solve_blocks > 0) {
+    if ((rc = enqueue_persistent_solve(S, s0, P, prof))) return rc;
+    gmres_finish_kernel<<<1, S.nthr, 0, s0>>>(I.gm, I.res, S.nslot, I.act);
+    return end_step(S, s0, prof, out);
+  }
   enqueue_solve_init(S, s0, P, gh);
   if ((rc = begin_conditional(c, s0, s1, gh.loop, cudaGraphCondTypeWhile))) return rc;
   for (int j = 0; j < o.gmres_restart; ++j) {
@@ -727,14 +848,7 @@ int capture_step(bes_ctx* c, int prof, cudaGraph_t* out) {
   enqueue_cycle_end(S, s1, P, gh);
   if ((rc = end_conditional(c, s1, &I.nodes_loop[prof]))) return rc;
   gmres_finish_kernel<<<1, S.nthr, 0, s0>>>(I.gm, I.res, S.nslot, I.act);
-  stamp(c, s0, PROF_OTHER, 1);
-  state_update_kernel<T><<<S.vgrid, 256, 0, s0>>>(slots(c->U[c->cur], 5LL * S.nc), S.cvec(S.X),
-                                                  (int64_t)S.nc, c->nan_flag, I.act);
-  stamp(c, s0, PROF_OTHER, 0);
-  IMP_TRY(c, cudaGetLastError());
-  IMP_TRY(c, cudaStreamEndCapture(s0, out));
-  I.nodes_top[prof] = kernel_nodes(*out);
-  return BES_OK;
+  return end_step(S, s0, prof, out);
 }
 
 template <class T, class B>
@@ -1101,6 +1215,13 @@ int implicit_allocate(bes_ctx* c) {
     else
       e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, ilu_sweep_persistent_kernel<double, false>, 128, 0);
     I.persistent_blocks = (coop && e == cudaSuccess) ? per_sm * sms : 0;
+    if (I.packed)
+      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, gmres_solve_kernel<float, __half, true>, 256, 0);
+    else if (I.prec)
+      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, gmres_solve_kernel<float, float, false>, 256, 0);
+    else
+      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, gmres_solve_kernel<double, double, false>, 256, 0);
+    I.solve_resident = (coop && e == cudaSuccess) ? per_sm * sms : 0;
     cudaGetLastError();
   }
   IMP_TRY(c, cudaMemset(I.res, 0, ns * sizeof(StepResult)));

@@ -88,16 +88,25 @@ __device__ __forceinline__ void load_packed_once(const __half2* __restrict__ H, 
 }
 
 // ---- gathers of a cell's five values ------------------------------------------------------------
+// Load of a Krylov vector entry; COH: through L2 only (ld.global.cg), for values that other
+// blocks of the same launch wrote (a persistent sweep or solve: L1 is not coherent across SMs).
+template <bool COH, class T>
+__device__ __forceinline__ T vld(const T* p) {
+  if constexpr (COH) return __ldcg(p);
+  else return *p;
+}
+
 // A Krylov vector holds a cell's five FP32 values in 20 consecutive bytes, which always lie in
-// two aligned 16-byte chunks.  Loading those two chunks takes two load instructions per
-// neighbour instead of five (for a warp whose neighbours are scattered, one L1 wavefront per
-// lane and instruction).  The vectors are 16-byte aligned and have at least 16 bytes after the
-// last cell of every slot (the vector stride), so both chunks are in bounds.  The values are
-// the same floats either way.
+// two aligned 16-byte chunks (FP64: 40 bytes in three).  Loading the chunks takes two (three)
+// load instructions per neighbour instead of five (for a warp whose neighbours are scattered,
+// one L1 wavefront per lane and instruction).  The vectors are 16-byte aligned and have at
+// least 16 bytes after the last cell of every slot (the vector stride), so every chunk is in
+// bounds.  The values are the same either way.
+template <bool COH = false>
 __device__ __forceinline__ void gather5(const float* __restrict__ x, int j, float* y) {
   const int64_t e0 = (int64_t)j * 5;
   const float4* p = reinterpret_cast<const float4*>(x) + (e0 >> 2);
-  const float4 a = p[0], b = p[1];
+  const float4 a = vld<COH>(p), b = vld<COH>(p + 1);
   const float w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
   const int o = (int)(e0 & 3);
 #pragma unroll
@@ -109,16 +118,23 @@ __device__ __forceinline__ void gather5(const float* __restrict__ x, int j, floa
     y[v] = t;
   }
 }
+template <bool COH = false>
+__device__ __forceinline__ void gather5(const double* __restrict__ x, int j, double* y) {
+  const int64_t e0 = (int64_t)j * 5;
+  const double2* p = reinterpret_cast<const double2*>(x) + (e0 >> 1);
+  const double2 a = vld<COH>(p), b = vld<COH>(p + 1), c = vld<COH>(p + 2);
+  const double w[6] = {a.x, a.y, b.x, b.y, c.x, c.y};
+  const bool odd = e0 & 1;
+#pragma unroll
+  for (int v = 0; v < 5; ++v) y[v] = odd ? w[v + 1] : w[v];
+}
+
+// Explicit fused multiply-add: where a sum of products starts from zero, the compiler may
+// contract a*a + b*b either way, and two kernels that must agree bit for bit might not.
+__device__ __forceinline__ float fma_t(float a, float b, float c) { return fmaf(a, b, c); }
+__device__ __forceinline__ double fma_t(double a, double b, double c) { return fma(a, b, c); }
 
 // ---- preconditioners ------------------------------------------------------------------------
-
-// Load of a Krylov vector entry; COH: through L2 only (ld.global.cg), for values that other
-// blocks of the same launch wrote (a persistent sweep: L1 is not coherent across SMs).
-template <bool COH, class T>
-__device__ __forceinline__ T vld(const T* p) {
-  if constexpr (COH) return __ldcg(p);
-  else return *p;
-}
 
 // Colour-ordered block-ILU(0) sweep when the colours are contiguous cell ranges in increasing
 // order (the colour-major numbering): the rows of one colour are [r0, r1), lower neighbours
@@ -135,15 +151,9 @@ __device__ __forceinline__ void ilu_colour_row(const DevMesh& m, int i, int r0, 
                                                const T* __restrict__ Dinv,
                                                const T* __restrict__ in, T* __restrict__ out) {
   const int nc = m.nc;
-  constexpr bool G = !COH && std::is_same<T, float>::value;  // two-chunk gathers
   const T* own = (LOWER || r0 == 0) ? in : out;
   T acc[5];
-  if constexpr (G) {
-    gather5(own, i, acc);
-  } else {
-#pragma unroll
-    for (int v = 0; v < 5; ++v) acc[v] = vld<COH>(own + (int64_t)i * 5 + v);
-  }
+  gather5<COH>(own, i, acc);
 #pragma unroll
   for (int s = 0; s < 4; ++s) {
     const int j = m.adj[s * nc + i];
@@ -152,23 +162,18 @@ __device__ __forceinline__ void ilu_colour_row(const DevMesh& m, int i, int r0, 
     if (!lower && !upper) continue;
     const T* src = (lower && j < s1) ? in : out;
     T y[5];
-    if constexpr (G) {
-      gather5(src, j, y);
-    } else {
-#pragma unroll
-      for (int v = 0; v < 5; ++v) y[v] = vld<COH>(src + (int64_t)j * 5 + v);
-    }
+    gather5<COH>(src, j, y);
 #pragma unroll
     for (int r = 0; r < 5; ++r)
 #pragma unroll
-      for (int c = 0; c < 5; ++c) acc[r] -= ellc(A, 1 + s, r * 5 + c, nc, i) * y[c];
+      for (int c = 0; c < 5; ++c) acc[r] = fma_t(-ellc(A, 1 + s, r * 5 + c, nc, i), y[c], acc[r]);
   }
   if (UPPER) {
 #pragma unroll
     for (int r = 0; r < 5; ++r) {
       T x = T(0);
 #pragma unroll
-      for (int c = 0; c < 5; ++c) x += Dinv[(int64_t)(r * 5 + c) * nc + i] * acc[c];
+      for (int c = 0; c < 5; ++c) x = fma_t(Dinv[(int64_t)(r * 5 + c) * nc + i], acc[c], x);
       out[(int64_t)i * 5 + r] = x;
     }
   } else {
@@ -197,12 +202,7 @@ __device__ __forceinline__ void ilu_colour_packed_row(
   const uint64_t pol = l2_evict_first();
   const float* own = (LOWER || r0 == 0) ? in : out;
   float acc[5];
-  if constexpr (!COH) {
-    gather5(own, i, acc);
-  } else {
-#pragma unroll
-    for (int v = 0; v < 5; ++v) acc[v] = vld<COH>(own + (int64_t)i * 5 + v);
-  }
+  gather5<COH>(own, i, acc);
   // the four neighbour ids first (one round trip), then the qualifying slots
   int jn[4];
 #pragma unroll
@@ -216,14 +216,9 @@ __device__ __forceinline__ void ilu_colour_packed_row(
     const float* src = (lower && j < s1) ? in : out;
     const float sc = ld_once(HS + (int64_t)s * nc + i, pol);
     float y[5], a[26];
-    if constexpr (!COH) {
-      gather5(src, j, y);
+    gather5<COH>(src, j, y);
 #pragma unroll
-      for (int v = 0; v < 5; ++v) y[v] *= sc;
-    } else {
-#pragma unroll
-      for (int v = 0; v < 5; ++v) y[v] = sc * vld<COH>(src + (int64_t)j * 5 + v);
-    }
+    for (int v = 0; v < 5; ++v) y[v] *= sc;
     load_packed_once(H, s, nc, i, a, pol);
 #pragma unroll
     for (int r = 0; r < 5; ++r)
@@ -266,7 +261,7 @@ __global__ void __launch_bounds__(128) ilu_colour_packed_kernel(
 // (neighbour ids, then everything else) instead of one per qualifying slot, at the cost of
 // registers.  The arithmetic is that of ilu_colour_packed_row in the same order, so the
 // results are identical; the autotuner keeps it only where it is faster.
-template <bool LOWER, bool UPPER>
+template <bool LOWER, bool UPPER, bool COH = false>
 __device__ __forceinline__ void ilu_colour_packed_row_ld(
     const DevMesh& m, int i, int r0, int r1, int s1, const __half2* __restrict__ H,
     const float* __restrict__ HS, const __half2* __restrict__ D, const float* __restrict__ DS,
@@ -278,7 +273,7 @@ __device__ __forceinline__ void ilu_colour_packed_row_ld(
 #pragma unroll
   for (int s = 0; s < 4; ++s) jn[s] = m.adj[s * nc + i];
   float acc[5];
-  gather5(own, i, acc);
+  gather5<COH>(own, i, acc);
   bool q[4];
   __half2 hb[4][13];
   float sc[4], y[4][5];
@@ -293,7 +288,7 @@ __device__ __forceinline__ void ilu_colour_packed_row_ld(
       sc[s] = ld_once(HS + (int64_t)s * nc + i, pol);
 #pragma unroll
       for (int p = 0; p < 13; ++p) hb[s][p] = ld_once(H + (int64_t)(s * 13 + p) * nc + i, pol);
-      gather5(src, j, y[s]);
+      gather5<COH>(src, j, y[s]);
     }
   }
 #pragma unroll
@@ -548,18 +543,11 @@ __global__ void __launch_bounds__(256) copy_vec_kernel(SlotPtr<T> outp, SlotPtr<
 }
 
 // block-Jacobi application: out_i = Dinv_i in_i
-template <class T>
-__global__ void __launch_bounds__(256) jacobi_apply_kernel(int nc, SlotPtr<const T> Dp,
-                                                           SlotPtr<const T> inp, SlotPtr<T> outp,
-                                                           const int32_t* run) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nc || slot_idle(run)) return;
-  const T* __restrict__ Dinv = Dp.at();
-  const T* __restrict__ in = inp.at();
-  T* __restrict__ out = outp.at();
+template <class T, bool COH>
+__device__ __forceinline__ void jacobi_row(int nc, int i, const T* __restrict__ Dinv, const T* in,
+                                           T* out) {
   T x[5];
-#pragma unroll
-  for (int v = 0; v < 5; ++v) x[v] = in[(int64_t)i * 5 + v];
+  gather5<COH>(in, i, x);
 #pragma unroll
   for (int r = 0; r < 5; ++r) {
     T acc = T(0);
@@ -568,20 +556,24 @@ __global__ void __launch_bounds__(256) jacobi_apply_kernel(int nc, SlotPtr<const
     out[(int64_t)i * 5 + r] = acc;
   }
 }
-
-// block-Jacobi application with a packed inverse diagonal
-static __global__ void __launch_bounds__(256) jacobi_apply_packed_kernel(
-    int nc, SlotPtr<const __half2> Dp, SlotPtr<const float> DSp, SlotPtr<const float> inp,
-    SlotPtr<float> outp, const int32_t* run) {
+template <class T>
+__global__ void __launch_bounds__(256) jacobi_apply_kernel(int nc, SlotPtr<const T> Dp,
+                                                           SlotPtr<const T> inp, SlotPtr<T> outp,
+                                                           const int32_t* run) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= nc || slot_idle(run)) return;
-  const float* __restrict__ in = inp.at();
-  float* __restrict__ out = outp.at();
+  jacobi_row<T, false>(nc, i, Dp.at(), inp.at(), outp.at());
+}
+
+// block-Jacobi application with a packed inverse diagonal
+template <bool COH>
+__device__ __forceinline__ void jacobi_packed_row(int nc, int i, const __half2* __restrict__ D,
+                                                  const float* __restrict__ DS, const float* in,
+                                                  float* out) {
   float x[5], a[26];
-#pragma unroll
-  for (int v = 0; v < 5; ++v) x[v] = in[(int64_t)i * 5 + v];
-  load_packed(Dp.at(), 0, nc, i, a);
-  const float sc = DSp.at()[i];
+  gather5<COH>(in, i, x);
+  load_packed(D, 0, nc, i, a);
+  const float sc = DS[i];
 #pragma unroll
   for (int r = 0; r < 5; ++r) {
     float acc = 0.0f;
@@ -590,29 +582,23 @@ static __global__ void __launch_bounds__(256) jacobi_apply_packed_kernel(
     out[(int64_t)i * 5 + r] = sc * acc;
   }
 }
+static __global__ void __launch_bounds__(256) jacobi_apply_packed_kernel(
+    int nc, SlotPtr<const __half2> Dp, SlotPtr<const float> DSp, SlotPtr<const float> inp,
+    SlotPtr<float> outp, const int32_t* run) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= nc || slot_idle(run)) return;
+  jacobi_packed_row<false>(nc, i, Dp.at(), DSp.at(), inp.at(), outp.at());
+}
 
 // ---- matrix-vector products ------------------------------------------------------------------
 
-// y = A x (ELL), or y = b - A x when b is given
-template <class T, bool BATCH>
-__global__ void __launch_bounds__(256) spmv_kernel(DevMesh m, SlotPtr<const T> Ap,
-                                                   SlotPtr<const T> xp, SlotPtr<const T> bp,
-                                                   SlotPtr<T> yp, const int32_t* run) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+// Row i of y = A x (ELL), or y = b - A x when b is given
+template <class T, bool COH>
+__device__ __forceinline__ void spmv_row(const DevMesh& m, int i, const T* __restrict__ A,
+                                         const T* x, const T* __restrict__ b, T* y) {
   const int nc = m.nc;
-  if (i >= nc || slot_idle(run)) return;
-  const T* __restrict__ A = sat<BATCH>(Ap);
-  const T* __restrict__ x = sat<BATCH>(xp);
-  const T* __restrict__ b = bp.p ? sat<BATCH>(bp) : nullptr;
-  T* __restrict__ y = sat<BATCH>(yp);
-  constexpr bool G = std::is_same<T, float>::value;  // two-chunk gathers
   T acc[5], xi[5];
-  if constexpr (G) {
-    gather5(x, i, xi);
-  } else {
-#pragma unroll
-    for (int v = 0; v < 5; ++v) xi[v] = x[(int64_t)i * 5 + v];
-  }
+  gather5<COH>(x, i, xi);
 #pragma unroll
   for (int r = 0; r < 5; ++r) {
     T s = T(0);
@@ -624,12 +610,7 @@ __global__ void __launch_bounds__(256) spmv_kernel(DevMesh m, SlotPtr<const T> A
   for (int q = 0; q < 4; ++q) {
     const int j = m.adj[q * nc + i];
     if (j < 0) continue;
-    if constexpr (G) {
-      gather5(x, j, xi);
-    } else {
-#pragma unroll
-      for (int v = 0; v < 5; ++v) xi[v] = x[(int64_t)j * 5 + v];
-    }
+    gather5<COH>(x, j, xi);
 #pragma unroll
     for (int r = 0; r < 5; ++r)
 #pragma unroll
@@ -639,21 +620,23 @@ __global__ void __launch_bounds__(256) spmv_kernel(DevMesh m, SlotPtr<const T> A
   for (int r = 0; r < 5; ++r)
     y[(int64_t)i * 5 + r] = b ? b[(int64_t)i * 5 + r] - acc[r] : acc[r];
 }
-
-// y = A x (or b - A x) with A in packed form: per block, the neighbour's values are scaled
-// by the block's scale and multiplied by the 16-bit entries
-template <bool BATCH>
-__global__ void __launch_bounds__(256) spmv_packed_kernel(
-    DevMesh m, SlotPtr<const __half2> Hp, SlotPtr<const float> Sp, SlotPtr<const float> xp,
-    SlotPtr<const float> bp, SlotPtr<float> yp, const int32_t* run) {
+template <class T, bool BATCH>
+__global__ void __launch_bounds__(256) spmv_kernel(DevMesh m, SlotPtr<const T> Ap,
+                                                   SlotPtr<const T> xp, SlotPtr<const T> bp,
+                                                   SlotPtr<T> yp, const int32_t* run) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= m.nc || slot_idle(run)) return;
+  spmv_row<T, false>(m, i, sat<BATCH>(Ap), sat<BATCH>(xp), bp.p ? sat<BATCH>(bp) : nullptr,
+                     sat<BATCH>(yp));
+}
+
+// Row i of y = A x (or b - A x) with A in packed form: per block, the neighbour's values are
+// scaled by the block's scale and multiplied by the 16-bit entries
+template <bool COH>
+__device__ __forceinline__ void spmv_packed_row(const DevMesh& m, int i, const __half2* __restrict__ H,
+                                                const float* __restrict__ S, const float* x,
+                                                const float* __restrict__ b, float* y) {
   const int nc = m.nc;
-  if (i >= nc || slot_idle(run)) return;
-  const __half2* __restrict__ H = sat<BATCH>(Hp);
-  const float* __restrict__ S = sat<BATCH>(Sp);
-  const float* __restrict__ x = sat<BATCH>(xp);
-  const float* __restrict__ b = bp.p ? sat<BATCH>(bp) : nullptr;
-  float* __restrict__ y = sat<BATCH>(yp);
   float acc[5] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
   // branch-free, so that every slot's loads can be in flight together: the block of a slot
   // without a neighbour is zero (boundary face, or the empty fourth slot of a triangle), and
@@ -670,7 +653,7 @@ __global__ void __launch_bounds__(256) spmv_packed_kernel(
   for (int s = 0; s < 5; ++s) {
     const float sc = ld_once(S + (int64_t)s * nc + i, pol);
     float xs[5], a[26];
-    gather5(x, jn[s], xs);
+    gather5<COH>(x, jn[s], xs);
 #pragma unroll
     for (int v = 0; v < 5; ++v) xs[v] *= sc;
     load_packed_once(H, s, nc, i, a, pol);
@@ -682,6 +665,15 @@ __global__ void __launch_bounds__(256) spmv_packed_kernel(
 #pragma unroll
   for (int r = 0; r < 5; ++r)
     y[(int64_t)i * 5 + r] = b ? b[(int64_t)i * 5 + r] - acc[r] : acc[r];
+}
+template <bool BATCH>
+__global__ void __launch_bounds__(256) spmv_packed_kernel(
+    DevMesh m, SlotPtr<const __half2> Hp, SlotPtr<const float> Sp, SlotPtr<const float> xp,
+    SlotPtr<const float> bp, SlotPtr<float> yp, const int32_t* run) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= m.nc || slot_idle(run)) return;
+  spmv_packed_row<false>(m, i, sat<BATCH>(Hp), sat<BATCH>(Sp), sat<BATCH>(xp),
+                         bp.p ? sat<BATCH>(bp) : nullptr, sat<BATCH>(yp));
 }
 
 // ---- reductions ------------------------------------------------------------------------------
@@ -700,6 +692,43 @@ __device__ __forceinline__ A warp_sum_t(A x) {
   return x;
 }
 
+// Warp sums of M values at once (M <= 32): every step exchanges half of the values, so a lane
+// adds M - 1 times in all (plus one per step once a single value is left) instead of 5 M times.
+// Each value's sum is the same tree as warp_sum_t's, bit for bit; *pos receives the value whose
+// sum this lane holds in a[0], or -1.  With FP64 values (64 cycles an addition) the butterflies
+// of 16 sums took as long as the products of a 518,400-cell dot kernel.
+template <int M, int O, class A>
+__device__ __forceinline__ void warp_sums_step(A* a, int lane, int& pos, int& left) {
+  if constexpr (O > 0) {
+    if constexpr (M == 1) {
+      a[0] += __shfl_xor_sync(0xffffffffu, a[0], O);
+      if (lane & O) left = 0;  // the lane below holds the same sum
+      warp_sums_step<1, O / 2, A>(a, lane, pos, left);
+    } else {
+      constexpr int H = (M + 1) / 2;
+      const bool up = lane & O;
+#pragma unroll
+      for (int i = 0; i < H; ++i) {
+        const A hi = H + i < M ? a[H + i < M ? H + i : i] : A(0);
+        const A keep = up ? hi : a[i], send = up ? a[i] : hi;
+        a[i] = keep + __shfl_xor_sync(0xffffffffu, send, O);
+      }
+      // of the values this lane's half holds, `left` are not padding
+      pos += up ? H : 0;
+      left = up ? left - H : (left < H ? left : H);
+      warp_sums_step<H, O / 2, A>(a, lane, pos, left);
+    }
+  }
+}
+template <int M, class A>
+__device__ __forceinline__ int warp_sums(A* a) {
+  static_assert(M >= 1 && M <= 32, "one value per lane at the end");
+  const int lane = threadIdx.x & 31;
+  int pos = 0, left = M;
+  warp_sums_step<M, 16, A>(a, lane, pos, left);
+  return left > 0 ? pos : -1;
+}
+
 // Block reduction of NV per-thread accumulators; partials[k*gridDim.x + blk] (FP64).  Lanes
 // are summed in the accumulation type; each warp's sum is widened to FP64 once and the block's
 // eight warp sums are added in FP64 in a fixed order.
@@ -707,11 +736,13 @@ template <int NV, class A>
 __device__ __forceinline__ void block_reduce_store(A (&acc)[NV], double* partials) {
   __shared__ double sh[NV][8];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-#pragma unroll
-  for (int k = 0; k < NV; ++k) {
-    const A s = warp_sum_t<A>(acc[k]);
-    if (lane == 0) sh[k][wid] = (double)s;
+  constexpr int M = NV < 32 ? NV : 32;
+  if constexpr (NV > M) {
+    const A s = warp_sum_t<A>(acc[M]);
+    if (lane == 0) sh[M][wid] = (double)s;
   }
+  const int pos = warp_sums<M, A>(acc);
+  if (pos >= 0) sh[pos][wid] = (double)acc[0];
   __syncthreads();
   for (int k = threadIdx.x; k < NV; k += blockDim.x) {
     double s = 0.0;
@@ -893,7 +924,7 @@ __global__ void __launch_bounds__(256) gs_dots_kernel(SlotPtr<const B> Vp, int64
       for (int e = 0; e < P::W; ++e) wv[p * P::W + e] = (A)q.v[e];
     }
 #pragma unroll
-    for (int e = 0; e < W; ++e) acc[NV] += wv[e] * wv[e];
+    for (int e = 0; e < W; ++e) acc[NV] = fma_t(wv[e], wv[e], acc[NV]);
 #pragma unroll
     for (int k = 0; k < NV; ++k) {
       A vk[W];
@@ -905,7 +936,7 @@ __global__ void __launch_bounds__(256) gs_dots_kernel(SlotPtr<const B> Vp, int64
   if (blockIdx.x == 0 && threadIdx.x < N - ng * W) {  // the ragged tail, < W elements
     const int64_t i = ng * W + threadIdx.x;
     const A x = (A)w[i];
-    acc[NV] += x * x;
+    acc[NV] = fma_t(x, x, acc[NV]);
 #pragma unroll
     for (int k = 0; k < NV; ++k) acc[k] += IO::template get<A>(V + (int64_t)k * ldv, i) * x;
   }
@@ -938,7 +969,7 @@ static __global__ void gs_decide_kernel(SlotPtr<double> devp, SlotPtr<float> dev
   if (stage == 1) {
     const double nw2 = dev[nv];
     double s = 0.0;
-    for (int k = 0; k < nv; ++k) s += dev[k] * dev[k];
+    for (int k = 0; k < nv; ++k) s = fma(dev[k], dev[k], s);
     const double est = nw2 - s;
     const bool reorth = !(est > kReorthTheta2 * nw2);
     dev[kGsFlag] = reorth ? 1.0 : 0.0;
@@ -952,7 +983,7 @@ static __global__ void gs_decide_kernel(SlotPtr<double> devp, SlotPtr<float> dev
     if (dev[kGsFlag] == 0.0) return;
     const double nw2 = dev[kGsH2 + nv];
     double s = 0.0;
-    for (int k = 0; k < nv; ++k) s += dev[kGsH2 + k] * dev[kGsH2 + k];
+    for (int k = 0; k < nv; ++k) s = fma(dev[kGsH2 + k], dev[kGsH2 + k], s);
     const double e2 = nw2 - s;
     const double hn = e2 > 0.0 ? sqrt(e2) : 0.0;
     dev[kGsNorm] = hn;
@@ -1031,7 +1062,7 @@ __global__ void __launch_bounds__(256) gs_update_kernel(SlotPtr<B> outp, SlotPtr
         reinterpret_cast<P*>(w)[g * NP + p] = o;
       }
 #pragma unroll
-      for (int e = 0; e < W; ++e) acc[NV] += xr[e] * xr[e];
+      for (int e = 0; e < W; ++e) acc[NV] = fma_t(xr[e], xr[e], acc[NV]);
       // the second pass is rare: V is read again (from L2) for its dot products rather than
       // held in registers
 #pragma unroll
@@ -1065,7 +1096,7 @@ __global__ void __launch_bounds__(256) gs_update_kernel(SlotPtr<B> outp, SlotPtr
     if (MODE == GS_REORTH) {
       const T xt = (T)x;
       w[i] = xt;
-      acc[NV] += (A)xt * (A)xt;
+      acc[NV] = fma_t((A)xt, (A)xt, acc[NV]);
 #pragma unroll
       for (int k = 0; k < NV; ++k) acc[k] += IO::template get<A>(V + (int64_t)k * ldv, i) * (A)xt;
     } else {
@@ -1181,7 +1212,7 @@ __global__ void __launch_bounds__(256) norm2_kernel(SlotPtr<const T> xp, int64_t
   A sa = A(0);
   for (int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < N;
        idx += (int64_t)gridDim.x * blockDim.x)
-    sa += (A)x[idx] * (A)x[idx];
+    sa = fma_t((A)x[idx], (A)x[idx], sa);
   const double s = (double)warp_sum_t<A>(sa);
   if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = s;
   __syncthreads();
@@ -1256,35 +1287,39 @@ __device__ __forceinline__ void set_arnoldi_handles(const GmresHandles& h, int f
   for (int k = from; k < mr; ++k) cudaGraphSetConditional(h.arn[k], k == from ? first : 0u);
 }
 
-// Start of a solve: |b| (reduced into dev[kGsR]) gives beta; slots whose solve runs get
-// g = (beta, 0, ...), 1/beta for V_0 = b / beta, and both flags.
+// Start of slot t's solve: |b|^2 = nb2 gives beta; g = (beta, 0, ...), 1/beta for V_0 = b / beta.
+// Returns 1 if the solve runs.
+__device__ __forceinline__ int gmres_init_slot(const GmresDev& g, const GmresParam& P, int t,
+                                               double nb2, int nan_flag) {
+  const double nb = sqrt(nb2);
+  const double eps = P.tol * nb;
+  double* sc = g.sc + 8 * t;
+  sc[0] = nb;
+  sc[1] = eps;
+  sc[2] = nb;
+  sc[3] = nb > 0.0 ? 1.0 / nb : 0.0;
+  sc[4] = nb;
+  // the reference's solver reports a relative residual of 0 for b = 0; a solve that stops
+  // before its first iteration keeps r = b
+  sc[5] = nb > 0.0 ? 1.0 : 0.0;
+  g.iter[t] = 0;
+  g.jc[t] = 0;
+  g.second[t] = 0;
+  g.status[t] = BES_OK;
+  g.cycles[t] = 0;
+  double* gg = g.g + (int64_t)t * (kMaxRestart + 1);
+  gg[0] = nb;
+  for (int k = 1; k <= P.mr; ++k) gg[k] = 0.0;
+  return (nan_flag == 0 && nb > 0.0 && !(nb < eps) && P.maxiter > 0) ? 1 : 0;
+}
+
+// Start of a solve: the slots taking the step (|b|^2 reduced into dev[kGsR]) get their flags.
 static __global__ void gmres_init_kernel(GmresDev g, GmresParam P, GmresHandles h, int nslot,
                                          const int32_t* __restrict__ act,
                                          const int* __restrict__ nan_flag) {
   const int t = threadIdx.x;
   int lin = 0;
-  if (t < nslot && act[t]) {
-    const double nb = sqrt(g.dev[(int64_t)t * kGsLd + kGsR]);
-    const double eps = P.tol * nb;
-    double* sc = g.sc + 8 * t;
-    sc[0] = nb;
-    sc[1] = eps;
-    sc[2] = nb;
-    sc[3] = nb > 0.0 ? 1.0 / nb : 0.0;
-    sc[4] = nb;
-    lin = (*nan_flag == 0 && nb > 0.0 && !(nb < eps) && P.maxiter > 0) ? 1 : 0;
-    // the reference's solver reports a relative residual of 0 for b = 0; a solve that stops
-    // before its first iteration keeps r = b
-    sc[5] = nb > 0.0 ? 1.0 : 0.0;
-    g.iter[t] = 0;
-    g.jc[t] = 0;
-    g.second[t] = 0;
-    g.status[t] = BES_OK;
-    g.cycles[t] = 0;
-    double* gg = g.g + (int64_t)t * (kMaxRestart + 1);
-    gg[0] = nb;
-    for (int k = 1; k <= P.mr; ++k) gg[k] = 0.0;
-  }
+  if (t < nslot && act[t]) lin = gmres_init_slot(g, P, t, g.dev[(int64_t)t * kGsLd + kGsR], *nan_flag);
   if (t < nslot) {
     g.lin[t] = lin;
     g.cyc[t] = lin;
@@ -1353,34 +1388,40 @@ static __global__ void gmres_solve_y_kernel(GmresDev g, int nslot) {
   }
 }
 
-// After x += M^{-1} V y and r = b - A x (|r|^2 reduced into dev[kGsR]): the slot's solve
-// stops at |r| <= eps or at the iteration limit; otherwise the next cycle starts from
-// V_0 = r / |r|.  guard: restart cycles after which a slot is stopped with BES_ERR_TIMEOUT
-// (<= 0: linear_solver_max_iter + 1, more than a running solve can take).
+// After x += M^{-1} V y and r = b - A x (|r|^2 = nr2): slot t's solve stops at |r| <= eps or at
+// the iteration limit; otherwise the next cycle starts from V_0 = r / |r|.  guard: restart
+// cycles after which a slot is stopped with BES_ERR_TIMEOUT (<= 0: linear_solver_max_iter + 1,
+// more than a running solve can take).  Returns 1 if the solve goes on.
+__device__ __forceinline__ int gmres_restart_slot(const GmresDev& g, const GmresParam& P, int t,
+                                                  double nr2, int guard) {
+  double* sc = g.sc + 8 * t;
+  const double nr = sqrt(nr2);
+  sc[4] = nr;
+  const int limit = guard > 0 ? guard : P.maxiter + 1;
+  const int cycles = ++g.cycles[t];
+  if (nr <= sc[1] || g.iter[t] >= P.maxiter) {
+    sc[5] = nr / sc[0];
+    return 0;
+  }
+  if (cycles >= limit) {
+    sc[5] = nr / sc[0];
+    g.status[t] = BES_ERR_TIMEOUT;
+    return 0;
+  }
+  sc[2] = nr;
+  sc[3] = 1.0 / nr;
+  double* gg = g.g + (int64_t)t * (kMaxRestart + 1);
+  gg[0] = nr;
+  for (int k = 1; k <= P.mr; ++k) gg[k] = 0.0;
+  g.jc[t] = 0;
+  return 1;
+}
 static __global__ void gmres_restart_kernel(GmresDev g, GmresParam P, GmresHandles h, int nslot,
                                             const int32_t* __restrict__ guard) {
   const int t = threadIdx.x;
   int lin = 0;
   if (t < nslot && g.lin[t]) {
-    double* sc = g.sc + 8 * t;
-    const double nr = sqrt(g.dev[(int64_t)t * kGsLd + kGsR]);
-    sc[4] = nr;
-    const int limit = *guard > 0 ? *guard : P.maxiter + 1;
-    const int cycles = ++g.cycles[t];
-    if (nr <= sc[1] || g.iter[t] >= P.maxiter) {
-      sc[5] = nr / sc[0];
-    } else if (cycles >= limit) {
-      sc[5] = nr / sc[0];
-      g.status[t] = BES_ERR_TIMEOUT;
-    } else {
-      sc[2] = nr;
-      sc[3] = 1.0 / nr;
-      double* gg = g.g + (int64_t)t * (kMaxRestart + 1);
-      gg[0] = nr;
-      for (int k = 1; k <= P.mr; ++k) gg[k] = 0.0;
-      g.jc[t] = 0;
-      lin = 1;
-    }
+    lin = gmres_restart_slot(g, P, t, g.dev[(int64_t)t * kGsLd + kGsR], *guard);
     g.lin[t] = lin;
     g.cyc[t] = lin;
   }

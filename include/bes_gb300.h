@@ -154,7 +154,8 @@ int bes_explicit_iterations(bes_ctx* ctx, int64_t n, double* history);
  * CFL control (adaptive as adaptCourantNum_, src/SolverImplicit.cpp:530-550, or the additive
  * geometric ramp).  One step of every active condition is one CUDA graph launch: the GMRES
  * iteration (Arnoldi steps, Givens rotations, restarts, convergence test) runs on the device
- * inside the graph's conditional nodes, and the host synchronises once per step.
+ * inside the graph (its conditional nodes, or one persistent kernel on small meshes), and the
+ * host synchronises once per step.
  * history (may be NULL): [n][19] = L2[5] and max[5] of the Dt/V-scaled
  * right-hand side (the max is what the reference logs, Q10), CFL used, CFL after the step,
  * linear iterations, final relative linear residual, L2[5] of the unscaled residual
