@@ -128,15 +128,19 @@ __device__ __forceinline__ bool mbar_wait(uint32_t mbar, uint32_t parity) {
 }
 
 // Stage rows r0 .. r0 + rows - 1, values k0 .. k0 + K - 1 of src [..][ld] into sm (not waited for).
+// KC: K where it is known at compile time (the index arithmetic of a piece is then shifts), or 0.
+template <int KC>
 __device__ __forceinline__ void stage_async(uint32_t sm, const bf16* __restrict__ src, int64_t ld,
                                             int64_t r0, int rows, int64_t k0, int K) {
-  const int per = K / 8;
+  const int per = KC ? KC / 8 : K / 8;
+  const bf16* base = src + r0 * ld + k0;
+#pragma unroll 8
   for (int v = threadIdx.x; v < rows * per; v += blockDim.x) {
     // eight consecutive threads take eight rows of one core matrix (128 consecutive bytes)
     const int r = (v / (8 * per)) * 8 + (v & 7), seg = (v >> 3) % per;
     const uint32_t dst = sm + (r >> 3) * (per * kCoreBytes) + seg * kCoreBytes + (r & 7) * 16;
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n"
-                 :: "r"(dst), "l"(src + (r0 + r) * ld + k0 + seg * 8) : "memory");
+                 :: "r"(dst), "l"(base + r * ld + seg * 8) : "memory");
   }
 }
 __device__ __forceinline__ void stage_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
@@ -255,7 +259,8 @@ struct ForwardArgs {
   int* err;
 };
 
-constexpr int kFwdThreads = 512;
+constexpr int kFwdThreads = 1024;
+constexpr int kFwdCols = kW / (kFwdThreads / 128);  // columns of a warp's epilogue
 constexpr int kSmW = kW * kW * 2, kSmA = kRowTile * kW * 2;
 constexpr int kSmFilm = 2 * kW * 12 * 4, kSmC = kRowTile * 3 * 4, kSmW4 = kOut * kW * 4;
 constexpr int kFwdSmem = kSmW + kSmA + kSmFilm + kSmC + kSmW4 + kRowTile * kOut * 4;
@@ -280,13 +285,19 @@ __global__ void __launch_bounds__(kFwdThreads, 1) mlp_forward_kernel(const __gri
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int64_t r0 = (int64_t)blockIdx.x * ROWS;
   const uint32_t uW = smem_u32(sW), uA = smem_u32(sA);
-  stage_async(uA, a.X, kK0, r0, ROWS, 0, kK0);
-  stage_async(uW, a.Wb[0], kK0, 0, kW, 0, kK0);
+  stage_async<kK0>(uA, a.X, kK0, r0, ROWS, 0, kK0);
+  stage_async<kK0>(uW, a.Wb[0], kK0, 0, kW, 0, kK0);
   stage_commit();
   auto load_layer = [&](int l) {
     if (tid < kW) {
       const Film f = load_film(a.p + a.L.b[l], a.p + a.L.F[l], a.p + a.L.g[l], tid);
       float* d = film + ((l & 1) * kW + tid) * 12;
+      if (!TRAIN) {
+        // one condition for every row: gamma and beta are the column's
+        reinterpret_cast<float4*>(d)[0] =
+            make_float4(f.bias, film_gamma(f, a.c3[0], a.c3[1], a.c3[2]), film_beta(f, a.c3[0], a.c3[1], a.c3[2]), 0.0f);
+        return;
+      }
       reinterpret_cast<float4*>(d)[0] = make_float4(f.bias, f.f0, f.f1, f.f2);
       reinterpret_cast<float4*>(d)[1] = make_float4(f.gj, f.e0, f.e1, f.e2);
       d[8] = f.bj;
@@ -296,7 +307,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) mlp_forward_kernel(const __gri
   for (int q = tid; q < ROWS * 3; q += kFwdThreads) sC[q] = TRAIN ? a.C[r0 * 3 + q] : a.c3[q % 3];
   for (int q = tid; q < kOut * kW; q += kFwdThreads) w4[q] = a.p[a.L.W[kLayers] + q];
   TensorCta t = tensor_open<kW>(&mbar, &tmem_base);
-  const int row = (warp & 3) * 32 + lane, col0 = (warp >> 2) * 64;
+  const int row = (warp & 3) * 32 + lane, col0 = (warp >> 2) * kFwdCols;
   bool ok = true;
   for (int l = 0; l < kLayers && ok; ++l) {
     const int K = l == 0 ? kK0 : kW;
@@ -304,7 +315,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) mlp_forward_kernel(const __gri
     ok = tensor_mma<kW>(t, uA, uW, K, false);
     if (!ok) break;
     if (l + 1 < kLayers) {
-      stage_async(uW, a.Wb[l + 1], kW, 0, kW, 0, kW);
+      stage_async<kW>(uW, a.Wb[l + 1], kW, 0, kW, 0, kW);
       stage_commit();
       load_layer(l + 1);
     }
@@ -312,7 +323,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) mlp_forward_kernel(const __gri
       const float c0 = sC[row * 3], c1 = sC[row * 3 + 1], c2 = sC[row * 3 + 2];
       const float* fl = film + (l & 1) * kW * 12;
 #pragma unroll 1
-      for (int cc = 0; cc < 64; cc += 16) {
+      for (int cc = 0; cc < kFwdCols; cc += 16) {
         float x[16];
         tensor_read16(t, col0 + cc, x);
         uint32_t packed[8];
@@ -320,10 +331,14 @@ __global__ void __launch_bounds__(kFwdThreads, 1) mlp_forward_kernel(const __gri
         for (int q = 0; q < 16; ++q) {
           const int j = col0 + cc + q;
           const float4 fa = reinterpret_cast<const float4*>(fl + j * 12)[0];
-          const float4 fb = reinterpret_cast<const float4*>(fl + j * 12)[1];
-          const Film f{fa.y, fa.z, fa.w, fb.y, fb.z, fb.w, fb.x, fl[j * 12 + 8], fa.x};
-          const float gam = film_gamma(f, c0, c1, c2), bet = film_beta(f, c0, c1, c2);
-          const float z = x[q] + f.bias;
+          float gam = fa.y, bet = fa.z;
+          if (TRAIN) {
+            const float4 fb = reinterpret_cast<const float4*>(fl + j * 12)[1];
+            const Film f{fa.y, fa.z, fa.w, fb.y, fb.z, fb.w, fb.x, fl[j * 12 + 8], fa.x};
+            gam = film_gamma(f, c0, c1, c2);
+            bet = film_beta(f, c0, c1, c2);
+          }
+          const float z = x[q] + fa.x;
           const float y = z * (1.0f + gam) + bet;
           const bf16 h = __float2bfloat16(silu(y));
           if (TRAIN) {
@@ -393,8 +408,8 @@ __global__ void __launch_bounds__(256, 1) mlp_dh_kernel(const bf16* __restrict__
   const int64_t r0 = (int64_t)blockIdx.y * kRowTile;
   const int n0 = blockIdx.x * 128;
   const uint32_t uA = smem_u32(sm), uB = uA + kRowTile * kW * 2;
-  stage_async(uA, dZ, kW, r0, kRowTile, 0, kW);
-  stage_async(uB, WT, kW, n0, 128, 0, kW);
+  stage_async<kW>(uA, dZ, kW, r0, kRowTile, 0, kW);
+  stage_async<kW>(uB, WT, kW, n0, 128, 0, kW);
   stage_commit();
   TensorCta t = tensor_open<128>(&mbar, &tmem_base);
   stage_wait();
@@ -440,8 +455,13 @@ __global__ void __launch_bounds__(256, 1) mlp_dw_kernel(const __grid_constant__ 
   bool ok = true;
   for (int64_t k0 = k_begin; k0 < k_end && ok; k0 += kDwSlice) {
     const int n = (int)(k_end - k0 < kDwSlice ? k_end - k0 : kDwSlice);
-    stage_async(uA, a.dZT[l], a.ldt, m0, 128, k0, n);
-    stage_async(uB, a.HT[l], a.ldt, n0, 64, k0, n);
+    if (n == kDwSlice) {
+      stage_async<kDwSlice>(uA, a.dZT[l], a.ldt, m0, 128, k0, n);
+      stage_async<kDwSlice>(uB, a.HT[l], a.ldt, n0, 64, k0, n);
+    } else {
+      stage_async<0>(uA, a.dZT[l], a.ldt, m0, 128, k0, n);
+      stage_async<0>(uB, a.HT[l], a.ldt, n0, 64, k0, n);
+    }
     stage_commit();
     stage_wait();
     ok = tensor_mma<64>(t, uA, uB, n, k0 > k_begin);
@@ -681,16 +701,16 @@ struct UpdateArgs {
   int splits, chunks;
   float lr, wd, bc1, bc2;
 };
-// out = sum over q < n of src[q * stride], in increasing q, the loads eight at a time
+// out = sum over q < n of src[q * stride], in increasing q, the loads sixteen at a time
 __device__ __forceinline__ float sum_rows(const float* __restrict__ src, int64_t stride, int n) {
   float s = 0.0f;
   int q = 0;
-  for (; q + 8 <= n; q += 8) {
-    float x[8];
+  for (; q + 16 <= n; q += 16) {
+    float x[16];
 #pragma unroll
-    for (int e = 0; e < 8; ++e) x[e] = src[(q + e) * stride];
+    for (int e = 0; e < 16; ++e) x[e] = src[(q + e) * stride];
 #pragma unroll
-    for (int e = 0; e < 8; ++e) s += x[e];
+    for (int e = 0; e < 16; ++e) s += x[e];
   }
   for (; q < n; ++q) s += src[q * stride];
   return s;
