@@ -601,10 +601,9 @@ int bes_set_condition(bes_ctx* ctx, int32_t cond, const double* mach, const doub
                                  cudaMemcpyHostToDevice));
   }
   // the condition's state in reference numbering, or its step-0 freestream
-  std::vector<double> Uh(5 * nc);
-  if (U) {
-    std::copy(U, U + 5 * nc, Uh.begin());
-  } else {
+  std::vector<double> Uh;
+  if (!U) {
+    Uh.resize(5 * nc);
     double q[6];
     freestream_from(p, ctx->prm.ramp_steps, ctx->prm.ramp_frac, 0, q);
     double Uf[5];
@@ -618,7 +617,7 @@ int bes_set_condition(bes_ctx* ctx, int32_t cond, const double* mach, const doub
     for (int64_t i = 0; i < nc; ++i)
       for (int v = 0; v < 5; ++v) Uh[i * 5 + v] = Uf[v];
   }
-  BES_CUDA_TRY(ctx, cudaMemcpyAsync(ctx->stage, Uh.data(), 5 * nc * sizeof(double),
+  BES_CUDA_TRY(ctx, cudaMemcpyAsync(ctx->stage, U ? U : Uh.data(), 5 * nc * sizeof(double),
                                     cudaMemcpyHostToDevice, ctx->stream));
   state_from_stage_kernel<<<1024, 256, 0, ctx->stream>>>(
       (int)nc, 1, ctx->new2ref_dev, ctx->stage, ctx->U[ctx->cur] + (int64_t)cond * 5 * nc);

@@ -135,16 +135,12 @@ struct ImplicitBuffers {
   void* Z = nullptr;     // [ldv]
   void* W = nullptr;     // [ldv]
   void* X = nullptr;     // solution dW [ldv]
-  // precision 2: 16-bit block-scaled copies (half2 [slot][13][nc] + FP32 scale [slot][nc]) of
-  // A (5 slots), the off-diagonal ILU factors (4 slots) and the inverse diagonal (1 slot), per
-  // condition
+  // precision 2: 16-bit block-scaled copies (layout in implicit_kernels.cuh) of A (5 slots), the
+  // off-diagonal ILU factors (4 slots) and the inverse diagonal (1 slot), per condition
   bool packed = false;
-  void* A16 = nullptr;
-  float* As = nullptr;
-  void* LU16 = nullptr;
-  float* LUs = nullptr;
-  void* D16 = nullptr;
-  float* Ds = nullptr;
+  uint32_t* A16 = nullptr;
+  uint32_t* LU16 = nullptr;
+  uint32_t* D16 = nullptr;
   // precision 2: Krylov basis V in FP16 (kBasisScale times the value) and an FP32 copy of its
   // newest vector, the preconditioner's input
   bool basis16 = false;

@@ -32,8 +32,7 @@ struct SolveArgs {
   SweepPlan plan;       // colour stages (block ILU)
   SweepOps<T> ops;      // factors (block ILU) or inverse diagonal (block Jacobi)
   int ilu;
-  SlotPtr<const __half2> A16;  // packed matrix and scales
-  SlotPtr<const float> As;
+  SlotPtr<const uint32_t> A16;  // packed matrix
   SlotPtr<const T> A;          // matrix in T
   SlotPtr<const T> b;
   SlotPtr<T> Y, Z, W, X, Vx;
@@ -232,7 +231,7 @@ __device__ __forceinline__ void put_entry(T* x, T v) {
 // accumulated in the order of the row functions (slots, then columns).
 constexpr int kRowsPerWarp = 6;
 
-// A lane's words of one block row: five values of T, or three half2 of a packed block and its
+// A lane's words of one block row: five values of T, or three words of a packed block and its
 // scale (entries 5 r .. 5 r + 4 of the row-major block).
 template <class T, bool PACKED>
 struct LaneBlock {
@@ -246,19 +245,20 @@ struct LaneBlock {
 };
 template <>
 struct LaneBlock<float, true> {
-  __half2 w[3];
+  uint32_t w[3];
   float sc;
-  __device__ __forceinline__ void load(const __half2* __restrict__ H, const float* __restrict__ S, int s,
-                                       int nc, int i, int r) {
+  __device__ __forceinline__ void load(const uint32_t* __restrict__ H, int nslots, int s, int i, int r) {
+    const uint32_t* h = packed_slot(H, nslots, s, i);
     const int p0 = (5 * r) >> 1;
 #pragma unroll
-    for (int p = 0; p < 3; ++p) w[p] = H[(int64_t)(s * 13 + p0 + p) * nc + i];
-    sc = S[(int64_t)s * nc + i];
+    for (int p = 0; p < 3; ++p) w[p] = h[packed_word(p0 + p, i)];
+    sc = packed_scale(h[packed_word(12, i)]);
   }
   // entry c of the row: half 5 r + c of the block, and 5 r starts in the second half for odd r
   __device__ __forceinline__ float entry(int c, int r) const {
     const bool odd = r & 1;
-    const float2 even = __half22float2(w[c >> 1]), next = __half22float2(w[(c + 1) >> 1]);
+    const float2 even = __half22float2(*reinterpret_cast<const __half2*>(&w[c >> 1]));
+    const float2 next = __half22float2(*reinterpret_cast<const __half2*>(&w[(c + 1) >> 1]));
     const float e = (c & 1) ? even.y : even.x;         // half c of the words
     const float o = ((c + 1) & 1) ? next.y : next.x;   // half c + 1
     return odd ? o : e;
@@ -323,10 +323,10 @@ __device__ __forceinline__ void sweep_lane_load(const SolveArgs<T, B>& S, int st
 #pragma unroll
   for (int s = 0; s < 4; ++s) {
     L.j[s] = S.m.adj[s * nc + L.q.i];
-    if constexpr (PACKED) L.blk[s].load(S.ops.H.of(L.q.k), S.ops.HS.of(L.q.k), s, nc, L.q.i, r);
+    if constexpr (PACKED) L.blk[s].load(S.ops.H.of(L.q.k), 4, s, L.q.i, r);
     else L.blk[s].load(S.ops.L.of(L.q.k), 1 + s, nc, L.q.i, r);
   }
-  if constexpr (PACKED) L.inv.load(S.ops.D.of(L.q.k), S.ops.DS.of(L.q.k), 0, nc, L.q.i, r);
+  if constexpr (PACKED) L.inv.load(S.ops.D.of(L.q.k), 1, 0, L.q.i, r);
   else L.inv.load(S.ops.Dinv.of(L.q.k), 0, nc, L.q.i, r);
 }
 // One row of a stage by one component per lane (ilu_colour_row / ilu_colour_packed_row).  Every
@@ -386,7 +386,7 @@ __device__ __noinline__ void phase_jacobi(const SolveArgs<T, B>& S, const T* in,
     const RowItem q = row_item<true>(it, 0, nc, S.nslot, run);
     if (q.i < 0) continue;
     LaneBlock<T, PACKED> D;
-    if constexpr (PACKED) D.load(S.ops.D.of(q.k), S.ops.DS.of(q.k), 0, nc, q.i, r);
+    if constexpr (PACKED) D.load(S.ops.D.of(q.k), 1, 0, q.i, r);
     else D.load(S.ops.Dinv.of(q.k), 0, nc, q.i, r);
     T x[5], acc = T(0);
     gather5<true>(in + q.k * in_stride, q.i, x);
@@ -448,7 +448,7 @@ __device__ __noinline__ void phase_spmv(const SolveArgs<T, B>& S, const int* run
       LaneBlock<T, PACKED> blk[5];
 #pragma unroll
       for (int s = 0; s < 5; ++s) {
-        if constexpr (PACKED) blk[s].load(S.A16.of(q.k), S.As.of(q.k), s, nc, q.i, r);
+        if constexpr (PACKED) blk[s].load(S.A16.of(q.k), 5, s, q.i, r);
         else blk[s].load(S.A.of(q.k), s, nc, q.i, r);
       }
       const T* x = S.Z.of(q.k);
@@ -472,7 +472,7 @@ __device__ __noinline__ void phase_spmv(const SolveArgs<T, B>& S, const int* run
     if (q.i < 0) continue;
     if constexpr (RESIDUAL) {
       const T *x = S.X.of(q.k), *b = S.b.of(q.k);
-      if constexpr (PACKED) spmv_packed_row<true>(S.m, q.i, S.A16.of(q.k), S.As.of(q.k), x, b, S.W.of(q.k));
+      if constexpr (PACKED) spmv_packed_row<true>(S.m, q.i, S.A16.of(q.k), x, b, S.W.of(q.k));
       else spmv_row<T, true>(S.m, q.i, S.A.of(q.k), x, b, S.W.of(q.k));
     } else {
       const T* x = S.Z.of(q.k);
@@ -484,16 +484,15 @@ __device__ __noinline__ void phase_spmv(const SolveArgs<T, B>& S, const int* run
 #pragma unroll
       for (int s = 0; s < 5; ++s) {
         if (!PACKED && j[s] < 0) continue;
-        T a[26], y[5];
+        T a[25], y[5], sc = T(1);
         if constexpr (PACKED) {
-          load_packed(S.A16.of(q.k), s, nc, q.i, a);
+          sc = load_packed(S.A16.of(q.k), 5, s, q.i).unpack(a);
         } else {
 #pragma unroll
           for (int e = 0; e < 25; ++e) a[e] = ellc(S.A.of(q.k), s, e, nc, q.i);
         }
         wait_gather5(x, j[s] >= 0 ? j[s] : q.i, y, err);
         if constexpr (PACKED) {
-          const float sc = S.As.of(q.k)[(int64_t)s * nc + q.i];
 #pragma unroll
           for (int c = 0; c < 5; ++c) y[c] *= sc;
         }

@@ -69,8 +69,7 @@ struct Sys {
   T *A, *LU, *Dinv, *Dc, *b, *Z, *W, *X, *Vx;
   B* V;
   bool packed, basis16;
-  __half2 *A16, *LU16, *D16;
-  float *As, *LUs, *Ds;
+  uint32_t *A16, *LU16, *D16;
   cudaStream_t s;  // the stream being captured (switched inside conditional bodies)
   dim3 vgrid;      // vector kernels: kRedBlocks blocks per slot
   int nthr;        // control kernels: one thread per slot, rounded up to a warp
@@ -95,12 +94,9 @@ struct Sys {
     V = (B*)I.V;
     packed = I.packed;
     basis16 = I.basis16;
-    A16 = (__half2*)I.A16;
-    LU16 = (__half2*)I.LU16;
-    D16 = (__half2*)I.D16;
-    As = I.As;
-    LUs = I.LUs;
-    Ds = I.Ds;
+    A16 = I.A16;
+    LU16 = I.LU16;
+    D16 = I.D16;
     s = ctx->stream;
     vgrid = dim3(kRedBlocks, nslot);
     nthr = std::min(kMaxSlots, (nslot + 31) / 32 * 32);
@@ -110,6 +106,10 @@ struct Sys {
   SlotPtr<const T> cvec(const T* p) const { return cslots(p, ldv); }
   SlotPtr<B> basis(int k) const { return slots(V + (int64_t)k * ldv, sV); }
   SlotPtr<const B> cbasis(int k) const { return cslots(V + (int64_t)k * ldv, sV); }
+  // packed arrays: A (5 slots), the off-diagonal factors (4), the inverse diagonal (1)
+  SlotPtr<const uint32_t> packed_A() const { return cslots((const uint32_t*)A16, packed_words(nc, 5)); }
+  SlotPtr<const uint32_t> packed_LU() const { return cslots((const uint32_t*)LU16, packed_words(nc, 4)); }
+  SlotPtr<const uint32_t> packed_D() const { return cslots((const uint32_t*)D16, packed_words(nc, 1)); }
   SlotPtr<double> red() const { return slots(c->imp.red, 64 * c->imp.red_ld); }
   SlotPtr<const double> cred() const { return cslots(c->imp.red, 64 * c->imp.red_ld); }
   SlotPtr<double> dev(int off = 0) const { return slots(c->imp.gm.dev + off, (int64_t)kGsLd); }
@@ -210,10 +210,8 @@ SweepOps<T> sweep_ops(const Sys<T, B>& S) {
   SweepOps<T> O;
   std::memset(&O, 0, sizeof(O));
   if (S.packed) {
-    O.H = cslots((const __half2*)S.LU16, 52LL * S.nc);
-    O.HS = cslots((const float*)S.LUs, 4LL * S.nc);
-    O.D = cslots((const __half2*)S.D16, 13LL * S.nc);
-    O.DS = cslots((const float*)S.Ds, (int64_t)S.nc);
+    O.H = S.packed_LU();
+    O.D = S.packed_D();
   } else {
     O.L = cslots((const T*)S.LU, S.sA);
     O.Dinv = cslots((const T*)S.Dinv, S.sDinv);
@@ -264,8 +262,7 @@ int enqueue_persistent_solve(const Sys<T, B>& S, cudaStream_t s, const GmresPara
   if (a.ilu && !sweep_plan(c->soa, a.plan)) return BES_ERR_UNSUPPORTED;
   a.ops = sweep_ops(S);
   if (S.packed) {
-    a.A16 = cslots((const __half2*)S.A16, 65LL * S.nc);
-    a.As = cslots((const float*)S.As, 5LL * S.nc);
+    a.A16 = S.packed_A();
   } else {
     a.A = cslots((const T*)S.A, S.sA);
   }
@@ -323,8 +320,7 @@ void enqueue_precond(const Sys<T, B>& S, cudaStream_t s, SlotPtr<const T> in, co
     if constexpr (std::is_same<T, float>::value) {
       if (S.packed) {
         jacobi_apply_packed_kernel<<<dim3(nblk(S.nc, 256), S.nslot), 256, 0, s>>>(
-            S.nc, cslots((const __half2*)S.D16, 13LL * S.nc), cslots((const float*)S.Ds, (int64_t)S.nc),
-            in, Z, run);
+            S.nc, S.packed_D(), in, Z, run);
         return;
       }
     }
@@ -341,18 +337,13 @@ void enqueue_precond(const Sys<T, B>& S, cudaStream_t s, SlotPtr<const T> in, co
       const dim3 grid(nblk(r1 - r0, 128), S.nslot);
       if constexpr (std::is_same<T, float>::value) {
         if (S.packed) {
-          auto H = cslots((const __half2*)S.LU16, 52LL * S.nc);
-          auto HS = cslots((const float*)S.LUs, 4LL * S.nc);
-          auto D = cslots((const __half2*)S.D16, 13LL * S.nc);
-          auto DS = cslots((const float*)S.Ds, (int64_t)S.nc);
-#define BES_PACKED_SWEEP(LO, UP, BA)                                                          \
-  do {                                                                                        \
-    if (c->imp.sweep_kernel == 3)                                                             \
-      ilu_colour_packed_ld_kernel<LO, UP, BA><<<grid, 128, 0, s>>>(m, r0, r1, s1, H, HS, D, DS, \
-                                                                   in, Z, run);               \
-    else                                                                                      \
-      ilu_colour_packed_kernel<LO, UP, BA><<<grid, 128, 0, s>>>(m, r0, r1, s1, H, HS, D, DS,   \
-                                                                in, Z, run);                  \
+          const auto H = S.packed_LU(), D = S.packed_D();
+#define BES_PACKED_SWEEP(LO, UP, BA)                                                             \
+  do {                                                                                           \
+    if (c->imp.sweep_kernel == 3)                                                                \
+      ilu_colour_packed_ld_kernel<LO, UP, BA><<<grid, 128, 0, s>>>(m, r0, r1, s1, H, D, in, Z, run); \
+    else                                                                                         \
+      ilu_colour_packed_kernel<LO, UP, BA><<<grid, 128, 0, s>>>(m, r0, r1, s1, H, D, in, Z, run); \
   } while (0)
           if (S.nslot > 1) {
             if (lower && !upper) BES_PACKED_SWEEP(true, false, true);
@@ -410,12 +401,11 @@ void enqueue_spmv(const Sys<T, B>& S, cudaStream_t s, SlotPtr<const T> x, SlotPt
   const dim3 grid(nblk(S.nc, 256), S.nslot);
   if constexpr (std::is_same<T, float>::value) {
     if (S.packed) {
-      auto H = cslots((const __half2*)S.A16, 65LL * S.nc);
-      auto Sc = cslots((const float*)S.As, 5LL * S.nc);
+      const dim3 grid128(nblk(S.nc, 128), S.nslot);
       if (S.nslot > 1)
-        spmv_packed_kernel<true><<<grid, 256, 0, s>>>(S.c->dm, H, Sc, x, b, y, run);
+        spmv_packed_kernel<true><<<grid128, 128, 0, s>>>(S.c->dm, S.packed_A(), x, b, y, run);
       else
-        spmv_packed_kernel<false><<<grid, 256, 0, s>>>(S.c->dm, H, Sc, x, b, y, run);
+        spmv_packed_kernel<false><<<grid128, 128, 0, s>>>(S.c->dm, S.packed_A(), x, b, y, run);
       return;
     }
   }
@@ -543,9 +533,9 @@ void enqueue_residual_all(bes_ctx* c, cudaStream_t s, const SlotHandles& hs, int
 
 // 16-bit block-scaled copies (precision 2; T is float there)
 template <class T>
-void enqueue_pack(cudaStream_t s, int nc, const T* src, int slot0, int nslots, void* H, float* sc) {
+void enqueue_pack(cudaStream_t s, int nc, const T* src, int slot0, int nslots, uint32_t* H) {
   if constexpr (std::is_same<T, float>::value)
-    pack_blocks_kernel<<<dim3(nblk(nc, 256), nslots), 256, 0, s>>>(src, slot0, nc, (__half2*)H, sc);
+    pack_blocks_kernel<<<dim3(nblk(nc, 256), nslots), 256, 0, s>>>(src, slot0, nc, H);
 }
 
 // Slot k: first-order Jacobians, the assembled system with its right-hand side, the 16-bit
@@ -579,8 +569,8 @@ void enqueue_assembly(const Sys<T, B>& S, cudaStream_t s, int k, double* norms) 
                                              uses_ilu(c) ? nullptr : Dinv,
                                              c->imp.rhs + k * 5 * nc, S.b + k * S.ldv, red);
   if (S.packed) {
-    enqueue_pack(s, (int)nc, A, 0, 5, S.A16 + k * 65 * nc, S.As + k * 5 * nc);
-    if (!uses_ilu(c)) enqueue_pack(s, (int)nc, Dinv, 0, 1, S.D16 + k * 13 * nc, S.Ds + k * nc);
+    enqueue_pack(s, (int)nc, A, 0, 5, S.A16 + k * packed_words(nc, 5));
+    if (!uses_ilu(c)) enqueue_pack(s, (int)nc, Dinv, 0, 1, S.D16 + k * packed_words(nc, 1));
   }
   reduce_rows_kernel<<<15, 256, 0, s>>>(red, nb, 10, 1, norms);
   stamp(c, s, PROF_ASSEMBLE, 0);
@@ -614,8 +604,8 @@ void enqueue_factor(const Sys<T, B>& S, cudaStream_t s, int k) {
     }
   }
   if (S.packed) {
-    enqueue_pack(s, (int)nc, LU, 1, 4, S.LU16 + k * 52 * nc, S.LUs + k * 4 * nc);
-    enqueue_pack(s, (int)nc, Dinv, 0, 1, S.D16 + k * 13 * nc, S.Ds + k * nc);
+    enqueue_pack(s, (int)nc, LU, 1, 4, S.LU16 + k * packed_words(nc, 4));
+    enqueue_pack(s, (int)nc, Dinv, 0, 1, S.D16 + k * packed_words(nc, 1));
   }
   stamp(c, s, PROF_ILU_FACTOR, 0);
 }
@@ -659,9 +649,11 @@ void choose_solve(bes_ctx* c) {
 }
 
 // The colour-sweep variant, timed on this context's mesh and slots: one launch per colour, or
-// one persistent launch per sweep.  Each candidate runs 3 untimed and 10 timed sweeps (CUDA
-// events on the context's stream, all slots); a persistent candidate whose launch fails or
-// whose grid barrier gives up is dropped.  The options can fix the variant instead.
+// one persistent launch per sweep.  Each candidate runs 5 untimed and 10 timed sweeps of all slots
+// from a graph, as in the step (launched one by one on the stream, sweeps of fewer than 500,000
+// cells all took the 64 us that the launches take, and the persistent one was chosen where it
+// made the step 10 % slower); a persistent candidate whose launch fails or whose grid barrier
+// gives up is dropped.  The options can fix the variant instead.
 template <class T, class B>
 int tune_sweep(bes_ctx* c) {
   ImplicitBuffers& I = c->imp;
@@ -707,17 +699,28 @@ int tune_sweep(bes_ctx* c) {
     }
     if (cand == 3 && !I.packed) continue;  // a form of the 16-bit storage only
     I.sweep_kernel = cand;
-    bool ok = true;
     float ms = 0.0f;
-    for (int r = 0; r < 13 && ok; ++r) {
-      if (r == 3) cudaEventRecord(e0, c->stream);
+    // five sweeps as a graph, as the step runs them
+    cudaGraph_t graph = nullptr;
+    cudaGraphExec_t exec = nullptr;
+    IMP_TRY(c, cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeRelaxed));
+    bool ok = true;
+    for (int r = 0; r < 5 && ok; ++r) {
       if (cand == 2)
         ok = launch_persistent_sweep(S, c->stream, S.cvec(S.b), nullptr) == cudaSuccess;
       else
         enqueue_precond(S, c->stream, S.cvec(S.b), nullptr);
     }
+    ok = cudaStreamEndCapture(c->stream, &graph) == cudaSuccess && ok;
+    ok = ok && cudaGraphInstantiate(&exec, graph, 0) == cudaSuccess;
+    for (int r = 0; r < 3 && ok; ++r) {
+      if (r == 1) cudaEventRecord(e0, c->stream);
+      ok = cudaGraphLaunch(exec, c->stream) == cudaSuccess;
+    }
     cudaEventRecord(e1, c->stream);
     const cudaError_t e = cudaEventSynchronize(e1);
+    if (exec) cudaGraphExecDestroy(exec);
+    if (graph) cudaGraphDestroy(graph);
     if (e != cudaSuccess) {
       cudaEventDestroy(e0);
       cudaEventDestroy(e1);
@@ -1148,14 +1151,9 @@ int implicit_allocate(bes_ctx* c) {
   rc |= imp_malloc(c, &I.Dinv, 25 * nc * I.tsize * msl);
   if (uses_ilu(c)) rc |= imp_malloc(c, &I.LU, 125 * nc * I.tsize * msl);
   if (I.packed) {
-    rc |= imp_malloc(c, &I.A16, 65 * nc * sizeof(__half2) * ns);
-    rc |= imp_malloc(c, (void**)&I.As, 5 * nc * sizeof(float) * ns);
-    rc |= imp_malloc(c, &I.D16, 13 * nc * sizeof(__half2) * ns);
-    rc |= imp_malloc(c, (void**)&I.Ds, nc * sizeof(float) * ns);
-    if (uses_ilu(c)) {
-      rc |= imp_malloc(c, &I.LU16, 52 * nc * sizeof(__half2) * ns);
-      rc |= imp_malloc(c, (void**)&I.LUs, 4 * nc * sizeof(float) * ns);
-    }
+    rc |= imp_malloc(c, (void**)&I.A16, packed_words(nc, 5) * sizeof(uint32_t) * ns);
+    rc |= imp_malloc(c, (void**)&I.D16, packed_words(nc, 1) * sizeof(uint32_t) * ns);
+    if (uses_ilu(c)) rc |= imp_malloc(c, (void**)&I.LU16, packed_words(nc, 4) * sizeof(uint32_t) * ns);
   }
   rc |= imp_malloc(c, &I.Dc, 50 * nf * I.tsize);
   rc |= imp_malloc(c, &I.b, I.ldv * I.tsize * ns);

@@ -59,10 +59,10 @@ __device__ __forceinline__ uint64_t l2_evict_first() {
   asm("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
   return p;
 }
-__device__ __forceinline__ __half2 ld_once(const __half2* a, uint64_t pol) {
+__device__ __forceinline__ uint32_t ld_once(const uint32_t* a, uint64_t pol) {
   uint32_t v;
   asm("ld.global.nc.L2::cache_hint.b32 %0, [%1], %2;" : "=r"(v) : "l"(a), "l"(pol));
-  return *reinterpret_cast<const __half2*>(&v);
+  return v;
 }
 __device__ __forceinline__ float ld_once(const float* a, uint64_t pol) {
   float v;
@@ -77,14 +77,14 @@ __device__ __forceinline__ uint4 ld_once(const uint4* a, uint64_t pol) {
   return v;
 }
 // load_packed with the evict_first policy
-__device__ __forceinline__ void load_packed_once(const __half2* __restrict__ H, int s, int nc, int i,
-                                                 float* a, uint64_t pol) {
+__device__ __forceinline__ PackedBlock load_packed_once(const uint32_t* __restrict__ H, int nslots, int s,
+                                                        int i, uint64_t pol) {
+  const uint32_t* w = packed_slot(H, nslots, s, i);
+  PackedBlock b;
 #pragma unroll
-  for (int p = 0; p < 13; ++p) {
-    const float2 f = __half22float2(ld_once(H + (int64_t)(s * 13 + p) * nc + i, pol));
-    a[2 * p] = f.x;
-    a[2 * p + 1] = f.y;
-  }
+  for (int p = 0; p < 3; ++p) b.q[p] = ld_once(reinterpret_cast<const uint4*>(w + packed_word(4 * p, i)), pol);
+  b.last = ld_once(w + packed_word(12, i), pol);
+  return b;
 }
 
 // ---- gathers of a cell's five values ------------------------------------------------------------
@@ -195,9 +195,8 @@ __global__ void __launch_bounds__(128) ilu_colour_kernel(DevMesh m, int r0, int 
 
 template <bool LOWER, bool UPPER, bool COH = false>
 __device__ __forceinline__ void ilu_colour_packed_row(
-    const DevMesh& m, int i, int r0, int r1, int s1, const __half2* __restrict__ H,
-    const float* __restrict__ HS, const __half2* __restrict__ D, const float* __restrict__ DS,
-    const float* __restrict__ in, float* __restrict__ out) {
+    const DevMesh& m, int i, int r0, int r1, int s1, const uint32_t* __restrict__ H,
+    const uint32_t* __restrict__ D, const float* __restrict__ in, float* __restrict__ out) {
   const int nc = m.nc;
   const uint64_t pol = l2_evict_first();
   const float* own = (LOWER || r0 == 0) ? in : out;
@@ -214,21 +213,20 @@ __device__ __forceinline__ void ilu_colour_packed_row(
     const bool upper = UPPER && j >= r1;
     if (!lower && !upper) continue;
     const float* src = (lower && j < s1) ? in : out;
-    const float sc = ld_once(HS + (int64_t)s * nc + i, pol);
-    float y[5], a[26];
+    float y[5], a[25];
+    const PackedBlock blk = load_packed_once(H, 4, s, i, pol);
     gather5<COH>(src, j, y);
+    const float sc = blk.unpack(a);
 #pragma unroll
     for (int v = 0; v < 5; ++v) y[v] *= sc;
-    load_packed_once(H, s, nc, i, a, pol);
 #pragma unroll
     for (int r = 0; r < 5; ++r)
 #pragma unroll
       for (int c = 0; c < 5; ++c) acc[r] = fmaf(-a[r * 5 + c], y[c], acc[r]);
   }
   if (UPPER) {
-    float a[26];
-    load_packed_once(D, 0, nc, i, a, pol);
-    const float sc = ld_once(DS + i, pol);
+    float a[25];
+    const float sc = load_packed_once(D, 1, 0, i, pol).unpack(a);
 #pragma unroll
     for (int r = 0; r < 5; ++r) {
       float x = 0.0f;
@@ -245,15 +243,13 @@ __device__ __forceinline__ void ilu_colour_packed_row(
 // ilu_colour_kernel with packed factors: L / U blocks in H slots 0..3 (local faces 0..3),
 // inv(U_ii) in D (one slot)
 template <bool LOWER, bool UPPER, bool BATCH>
-__global__ void __launch_bounds__(128) ilu_colour_packed_kernel(
-    DevMesh m, int r0, int r1, int s1, SlotPtr<const __half2> Hp, SlotPtr<const float> HSp,
-    SlotPtr<const __half2> Dp, SlotPtr<const float> DSp, SlotPtr<const float> inp,
-    SlotPtr<float> outp, const int32_t* run) {
+__global__ void __launch_bounds__(128, 12) ilu_colour_packed_kernel(
+    DevMesh m, int r0, int r1, int s1, SlotPtr<const uint32_t> Hp, SlotPtr<const uint32_t> Dp,
+    SlotPtr<const float> inp, SlotPtr<float> outp, const int32_t* run) {
   const int i = r0 + blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= r1 || slot_idle(run)) return;
-  ilu_colour_packed_row<LOWER, UPPER>(m, i, r0, r1, s1, sat<BATCH>(Hp), sat<BATCH>(HSp),
-                                      sat<BATCH>(Dp), sat<BATCH>(DSp), sat<BATCH>(inp),
-                                      sat<BATCH>(outp));
+  ilu_colour_packed_row<LOWER, UPPER>(m, i, r0, r1, s1, sat<BATCH>(Hp), sat<BATCH>(Dp),
+                                      sat<BATCH>(inp), sat<BATCH>(outp));
 }
 
 // The packed colour sweep with every qualifying slot's loads (scale, 16-bit block, the
@@ -263,9 +259,8 @@ __global__ void __launch_bounds__(128) ilu_colour_packed_kernel(
 // results are identical; the autotuner keeps it only where it is faster.
 template <bool LOWER, bool UPPER, bool COH = false>
 __device__ __forceinline__ void ilu_colour_packed_row_ld(
-    const DevMesh& m, int i, int r0, int r1, int s1, const __half2* __restrict__ H,
-    const float* __restrict__ HS, const __half2* __restrict__ D, const float* __restrict__ DS,
-    const float* __restrict__ in, float* __restrict__ out) {
+    const DevMesh& m, int i, int r0, int r1, int s1, const uint32_t* __restrict__ H,
+    const uint32_t* __restrict__ D, const float* __restrict__ in, float* __restrict__ out) {
   const int nc = m.nc;
   const uint64_t pol = l2_evict_first();
   const float* own = (LOWER || r0 == 0) ? in : out;
@@ -275,8 +270,8 @@ __device__ __forceinline__ void ilu_colour_packed_row_ld(
   float acc[5];
   gather5<COH>(own, i, acc);
   bool q[4];
-  __half2 hb[4][13];
-  float sc[4], y[4][5];
+  PackedBlock blk[4];
+  float y[4][5];
 #pragma unroll
   for (int s = 0; s < 4; ++s) {
     const int j = jn[s];
@@ -285,33 +280,25 @@ __device__ __forceinline__ void ilu_colour_packed_row_ld(
     q[s] = lower || upper;
     if (q[s]) {
       const float* src = (lower && j < s1) ? in : out;
-      sc[s] = ld_once(HS + (int64_t)s * nc + i, pol);
-#pragma unroll
-      for (int p = 0; p < 13; ++p) hb[s][p] = ld_once(H + (int64_t)(s * 13 + p) * nc + i, pol);
+      blk[s] = load_packed_once(H, 4, s, i, pol);
       gather5<COH>(src, j, y[s]);
     }
   }
 #pragma unroll
   for (int s = 0; s < 4; ++s) {
     if (!q[s]) continue;
-    float a[26], ys[5];
+    float a[25], ys[5];
+    const float sc = blk[s].unpack(a);
 #pragma unroll
-    for (int p = 0; p < 13; ++p) {
-      const float2 f = __half22float2(hb[s][p]);
-      a[2 * p] = f.x;
-      a[2 * p + 1] = f.y;
-    }
-#pragma unroll
-    for (int v = 0; v < 5; ++v) ys[v] = sc[s] * y[s][v];
+    for (int v = 0; v < 5; ++v) ys[v] = sc * y[s][v];
 #pragma unroll
     for (int r = 0; r < 5; ++r)
 #pragma unroll
       for (int c = 0; c < 5; ++c) acc[r] = fmaf(-a[r * 5 + c], ys[c], acc[r]);
   }
   if (UPPER) {
-    float a[26];
-    load_packed_once(D, 0, nc, i, a, pol);
-    const float d = ld_once(DS + i, pol);
+    float a[25];
+    const float d = load_packed_once(D, 1, 0, i, pol).unpack(a);
 #pragma unroll
     for (int r = 0; r < 5; ++r) {
       float x = 0.0f;
@@ -327,14 +314,12 @@ __device__ __forceinline__ void ilu_colour_packed_row_ld(
 
 template <bool LOWER, bool UPPER, bool BATCH>
 __global__ void __launch_bounds__(128) ilu_colour_packed_ld_kernel(
-    DevMesh m, int r0, int r1, int s1, SlotPtr<const __half2> Hp, SlotPtr<const float> HSp,
-    SlotPtr<const __half2> Dp, SlotPtr<const float> DSp, SlotPtr<const float> inp,
-    SlotPtr<float> outp, const int32_t* run) {
+    DevMesh m, int r0, int r1, int s1, SlotPtr<const uint32_t> Hp, SlotPtr<const uint32_t> Dp,
+    SlotPtr<const float> inp, SlotPtr<float> outp, const int32_t* run) {
   const int i = r0 + blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= r1 || slot_idle(run)) return;
-  ilu_colour_packed_row_ld<LOWER, UPPER>(m, i, r0, r1, s1, sat<BATCH>(Hp), sat<BATCH>(HSp),
-                                         sat<BATCH>(Dp), sat<BATCH>(DSp), sat<BATCH>(inp),
-                                         sat<BATCH>(outp));
+  ilu_colour_packed_row_ld<LOWER, UPPER>(m, i, r0, r1, s1, sat<BATCH>(Hp), sat<BATCH>(Dp),
+                                         sat<BATCH>(inp), sat<BATCH>(outp));
 }
 
 // ---- persistent colour sweep ----------------------------------------------------------------
@@ -408,11 +393,10 @@ __device__ __forceinline__ bool grid_sync(const GridSync& g) {
   return ok != 0;
 }
 
-// Operands of a sweep: the factors (packed 16-bit with scales, or T) and the vectors.
+// Operands of a sweep: the factors (packed 16-bit, or T) and the vectors.
 template <class T>
 struct SweepOps {
-  SlotPtr<const __half2> H, D;   // packed: off-diagonal factor blocks, inverse diagonal
-  SlotPtr<const float> HS, DS;   // packed: their scales
+  SlotPtr<const uint32_t> H, D;  // packed: off-diagonal factor blocks, inverse diagonal
   SlotPtr<const T> L, Dinv;      // unpacked factors
   SlotPtr<const T> in;
   SlotPtr<T> out;
@@ -435,14 +419,14 @@ __global__ void __launch_bounds__(128) ilu_sweep_persistent_kernel(DevMesh m, Sw
       if (run != nullptr && run[k] == 0) continue;
       if constexpr (PACKED) {
         if (kind == 0)
-          ilu_colour_packed_row<true, false, true>(m, i, r0, r1, P.s1, O.H.of(k), O.HS.of(k),
-                                                   O.D.of(k), O.DS.of(k), O.in.of(k), O.out.of(k));
+          ilu_colour_packed_row<true, false, true>(m, i, r0, r1, P.s1, O.H.of(k), O.D.of(k),
+                                                  O.in.of(k), O.out.of(k));
         else if (kind == 1)
-          ilu_colour_packed_row<true, true, true>(m, i, r0, r1, P.s1, O.H.of(k), O.HS.of(k),
-                                                  O.D.of(k), O.DS.of(k), O.in.of(k), O.out.of(k));
+          ilu_colour_packed_row<true, true, true>(m, i, r0, r1, P.s1, O.H.of(k), O.D.of(k),
+                                                  O.in.of(k), O.out.of(k));
         else
-          ilu_colour_packed_row<false, true, true>(m, i, r0, r1, P.s1, O.H.of(k), O.HS.of(k),
-                                                   O.D.of(k), O.DS.of(k), O.in.of(k), O.out.of(k));
+          ilu_colour_packed_row<false, true, true>(m, i, r0, r1, P.s1, O.H.of(k), O.D.of(k),
+                                                  O.in.of(k), O.out.of(k));
       } else {
         if (kind == 0)
           ilu_colour_row<T, true, false, true>(m, i, r0, r1, P.s1, O.L.of(k), O.Dinv.of(k),
@@ -567,13 +551,12 @@ __global__ void __launch_bounds__(256) jacobi_apply_kernel(int nc, SlotPtr<const
 
 // block-Jacobi application with a packed inverse diagonal
 template <bool COH>
-__device__ __forceinline__ void jacobi_packed_row(int nc, int i, const __half2* __restrict__ D,
-                                                  const float* __restrict__ DS, const float* in,
+__device__ __forceinline__ void jacobi_packed_row(int i, const uint32_t* __restrict__ D, const float* in,
                                                   float* out) {
-  float x[5], a[26];
+  float x[5], a[25];
+  const PackedBlock blk = load_packed(D, 1, 0, i);
   gather5<COH>(in, i, x);
-  load_packed(D, 0, nc, i, a);
-  const float sc = DS[i];
+  const float sc = blk.unpack(a);
 #pragma unroll
   for (int r = 0; r < 5; ++r) {
     float acc = 0.0f;
@@ -583,11 +566,11 @@ __device__ __forceinline__ void jacobi_packed_row(int nc, int i, const __half2* 
   }
 }
 static __global__ void __launch_bounds__(256) jacobi_apply_packed_kernel(
-    int nc, SlotPtr<const __half2> Dp, SlotPtr<const float> DSp, SlotPtr<const float> inp,
-    SlotPtr<float> outp, const int32_t* run) {
+    int nc, SlotPtr<const uint32_t> Dp, SlotPtr<const float> inp, SlotPtr<float> outp,
+    const int32_t* run) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= nc || slot_idle(run)) return;
-  jacobi_packed_row<false>(nc, i, Dp.at(), DSp.at(), inp.at(), outp.at());
+  jacobi_packed_row<false>(i, Dp.at(), inp.at(), outp.at());
 }
 
 // ---- matrix-vector products ------------------------------------------------------------------
@@ -633,9 +616,8 @@ __global__ void __launch_bounds__(256) spmv_kernel(DevMesh m, SlotPtr<const T> A
 // Row i of y = A x (or b - A x) with A in packed form: per block, the neighbour's values are
 // scaled by the block's scale and multiplied by the 16-bit entries
 template <bool COH>
-__device__ __forceinline__ void spmv_packed_row(const DevMesh& m, int i, const __half2* __restrict__ H,
-                                                const float* __restrict__ S, const float* x,
-                                                const float* __restrict__ b, float* y) {
+__device__ __forceinline__ void spmv_packed_row(const DevMesh& m, int i, const uint32_t* __restrict__ H,
+                                                const float* x, const float* __restrict__ b, float* y) {
   const int nc = m.nc;
   float acc[5] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
   // branch-free, so that every slot's loads can be in flight together: the block of a slot
@@ -651,12 +633,12 @@ __device__ __forceinline__ void spmv_packed_row(const DevMesh& m, int i, const _
   const uint64_t pol = l2_evict_first();
 #pragma unroll
   for (int s = 0; s < 5; ++s) {
-    const float sc = ld_once(S + (int64_t)s * nc + i, pol);
-    float xs[5], a[26];
+    float xs[5], a[25];
+    const PackedBlock blk = load_packed_once(H, 5, s, i, pol);
     gather5<COH>(x, jn[s], xs);
+    const float sc = blk.unpack(a);
 #pragma unroll
     for (int v = 0; v < 5; ++v) xs[v] *= sc;
-    load_packed_once(H, s, nc, i, a, pol);
 #pragma unroll
     for (int r = 0; r < 5; ++r)
 #pragma unroll
@@ -666,14 +648,16 @@ __device__ __forceinline__ void spmv_packed_row(const DevMesh& m, int i, const _
   for (int r = 0; r < 5; ++r)
     y[(int64_t)i * 5 + r] = b ? b[(int64_t)i * 5 + r] - acc[r] : acc[r];
 }
+// Blocks of 128 with 12 of them resident: more loads in flight than the registers of a row that
+// the compiler would keep (2.16M cells: 129 us without the bound, 102 with 12 or 8, 125 with 16).
 template <bool BATCH>
-__global__ void __launch_bounds__(256) spmv_packed_kernel(
-    DevMesh m, SlotPtr<const __half2> Hp, SlotPtr<const float> Sp, SlotPtr<const float> xp,
-    SlotPtr<const float> bp, SlotPtr<float> yp, const int32_t* run) {
+__global__ void __launch_bounds__(128, 12) spmv_packed_kernel(
+    DevMesh m, SlotPtr<const uint32_t> Hp, SlotPtr<const float> xp, SlotPtr<const float> bp,
+    SlotPtr<float> yp, const int32_t* run) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= m.nc || slot_idle(run)) return;
-  spmv_packed_row<false>(m, i, sat<BATCH>(Hp), sat<BATCH>(Sp), sat<BATCH>(xp),
-                         bp.p ? sat<BATCH>(bp) : nullptr, sat<BATCH>(yp));
+  spmv_packed_row<false>(m, i, sat<BATCH>(Hp), sat<BATCH>(xp), bp.p ? sat<BATCH>(bp) : nullptr,
+                         sat<BATCH>(yp));
 }
 
 // ---- reductions ------------------------------------------------------------------------------
