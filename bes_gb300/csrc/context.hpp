@@ -121,11 +121,12 @@ struct ImplicitBuffers {
   size_t tsize = 8;      // sizeof(T)
   int nslot = 1;
   int64_t ldv = 0;       // Krylov vector stride: 5 nc rounded up to 64 elements
-  // system in T: ELL blocks [5 slots][25][nc]; per condition (precision 0/1) or one shared
-  // scratch (precision 2); sA etc. are the per-condition strides in elements (0: shared)
+  // system in T: blocks of 5 slots (layout in implicit_kernels.cuh); per condition (precision
+  // 0/1) or one shared scratch (precision 2); sA etc. are the per-condition strides in elements
+  // (0: shared)
   void* A = nullptr;
   void* LU = nullptr;    // block-ILU(0) factors in the same layout (ILU only)
-  void* Dinv = nullptr;  // [25][nc] inverse diagonal (Jacobi) / inverse U_ii (ILU)
+  void* Dinv = nullptr;  // 1 slot: inverse diagonal (Jacobi) / inverse U_ii (ILU)
   int64_t sA = 0, sDinv = 0;
   void* Dc = nullptr;    // per-face diagonal contributions [2][25][nf] (shared)
   // Krylov side, per condition

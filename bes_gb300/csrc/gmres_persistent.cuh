@@ -236,9 +236,11 @@ constexpr int kRowsPerWarp = 6;
 template <class T, bool PACKED>
 struct LaneBlock {
   T a[5];
-  __device__ __forceinline__ void load(const T* __restrict__ A, int s, int nc, int i, int r) {
+  __device__ __forceinline__ void load(const T* __restrict__ A, int nslots, int s, int i, int r) {
+    // (entry by entry: 16-byte words and selecting from them cost more than they save here)
+    const T* p = A + block_at<T>(nslots, s, 0, i - (i & 31));
 #pragma unroll
-    for (int c = 0; c < 5; ++c) a[c] = A[(int64_t)(s * 25 + r * 5 + c) * nc + i];
+    for (int c = 0; c < 5; ++c) a[c] = p[block_at<T>(1, 0, 5 * r + c, i & 31)];
   }
   __device__ __forceinline__ T entry(int c, int) const { return a[c]; }
   __device__ __forceinline__ T scale() const { return T(1); }
@@ -324,10 +326,10 @@ __device__ __forceinline__ void sweep_lane_load(const SolveArgs<T, B>& S, int st
   for (int s = 0; s < 4; ++s) {
     L.j[s] = S.m.adj[s * nc + L.q.i];
     if constexpr (PACKED) L.blk[s].load(S.ops.H.of(L.q.k), 4, s, L.q.i, r);
-    else L.blk[s].load(S.ops.L.of(L.q.k), 1 + s, nc, L.q.i, r);
+    else L.blk[s].load(S.ops.L.of(L.q.k), 5, 1 + s, L.q.i, r);
   }
   if constexpr (PACKED) L.inv.load(S.ops.D.of(L.q.k), 1, 0, L.q.i, r);
-  else L.inv.load(S.ops.Dinv.of(L.q.k), 0, nc, L.q.i, r);
+  else L.inv.load(S.ops.Dinv.of(L.q.k), 1, 0, L.q.i, r);
 }
 // One row of a stage by one component per lane (ilu_colour_row / ilu_colour_packed_row).  Every
 // lane of the warp calls.
@@ -387,7 +389,7 @@ __device__ __noinline__ void phase_jacobi(const SolveArgs<T, B>& S, const T* in,
     if (q.i < 0) continue;
     LaneBlock<T, PACKED> D;
     if constexpr (PACKED) D.load(S.ops.D.of(q.k), 1, 0, q.i, r);
-    else D.load(S.ops.Dinv.of(q.k), 0, nc, q.i, r);
+    else D.load(S.ops.Dinv.of(q.k), 1, 0, q.i, r);
     T x[5], acc = T(0);
     gather5<true>(in + q.k * in_stride, q.i, x);
 #pragma unroll
@@ -449,7 +451,7 @@ __device__ __noinline__ void phase_spmv(const SolveArgs<T, B>& S, const int* run
 #pragma unroll
       for (int s = 0; s < 5; ++s) {
         if constexpr (PACKED) blk[s].load(S.A16.of(q.k), 5, s, q.i, r);
-        else blk[s].load(S.A.of(q.k), s, nc, q.i, r);
+        else blk[s].load(S.A.of(q.k), 5, s, q.i, r);
       }
       const T* x = S.Z.of(q.k);
       T acc = T(0);
@@ -488,8 +490,7 @@ __device__ __noinline__ void phase_spmv(const SolveArgs<T, B>& S, const int* run
         if constexpr (PACKED) {
           sc = load_packed(S.A16.of(q.k), 5, s, q.i).unpack(a);
         } else {
-#pragma unroll
-          for (int e = 0; e < 25; ++e) a[e] = ellc(S.A.of(q.k), s, e, nc, q.i);
+          load_block(S.A.of(q.k), 5, s, q.i, a);
         }
         wait_gather5(x, j[s] >= 0 ? j[s] : q.i, y, err);
         if constexpr (PACKED) {

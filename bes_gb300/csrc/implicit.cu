@@ -398,21 +398,20 @@ void enqueue_precond(const Sys<T, B>& S, cudaStream_t s, SlotPtr<const T> in, co
 template <class T, class B>
 void enqueue_spmv(const Sys<T, B>& S, cudaStream_t s, SlotPtr<const T> x, SlotPtr<const T> b,
                   SlotPtr<T> y, const int32_t* run) {
-  const dim3 grid(nblk(S.nc, 256), S.nslot);
+  const dim3 grid(nblk(S.nc, 128), S.nslot);
   if constexpr (std::is_same<T, float>::value) {
     if (S.packed) {
-      const dim3 grid128(nblk(S.nc, 128), S.nslot);
       if (S.nslot > 1)
-        spmv_packed_kernel<true><<<grid128, 128, 0, s>>>(S.c->dm, S.packed_A(), x, b, y, run);
+        spmv_packed_kernel<true><<<grid, 128, 0, s>>>(S.c->dm, S.packed_A(), x, b, y, run);
       else
-        spmv_packed_kernel<false><<<grid128, 128, 0, s>>>(S.c->dm, S.packed_A(), x, b, y, run);
+        spmv_packed_kernel<false><<<grid, 128, 0, s>>>(S.c->dm, S.packed_A(), x, b, y, run);
       return;
     }
   }
   if (S.nslot > 1)
-    spmv_kernel<T, true><<<grid, 256, 0, s>>>(S.c->dm, cslots((const T*)S.A, S.sA), x, b, y, run);
+    spmv_kernel<T, true><<<grid, 128, 0, s>>>(S.c->dm, cslots((const T*)S.A, S.sA), x, b, y, run);
   else
-    spmv_kernel<T, false><<<grid, 256, 0, s>>>(S.c->dm, cslots((const T*)S.A, S.sA), x, b, y, run);
+    spmv_kernel<T, false><<<grid, 128, 0, s>>>(S.c->dm, cslots((const T*)S.A, S.sA), x, b, y, run);
 }
 
 // Body of the IF node of Arnoldi step j (slots with a running cycle): w = A M^{-1} v_j,
@@ -533,9 +532,10 @@ void enqueue_residual_all(bes_ctx* c, cudaStream_t s, const SlotHandles& hs, int
 
 // 16-bit block-scaled copies (precision 2; T is float there)
 template <class T>
-void enqueue_pack(cudaStream_t s, int nc, const T* src, int slot0, int nslots, uint32_t* H) {
+void enqueue_pack(cudaStream_t s, int nc, const T* src, int src_slots, int slot0, int nslots,
+                  uint32_t* H) {
   if constexpr (std::is_same<T, float>::value)
-    pack_blocks_kernel<<<dim3(nblk(nc, 256), nslots), 256, 0, s>>>(src, slot0, nc, H);
+    pack_blocks_kernel<<<dim3(nblk(nc, 256), nslots), 256, 0, s>>>(src, src_slots, slot0, nc, H);
 }
 
 // Slot k: first-order Jacobians, the assembled system with its right-hand side, the 16-bit
@@ -569,8 +569,8 @@ void enqueue_assembly(const Sys<T, B>& S, cudaStream_t s, int k, double* norms) 
                                              uses_ilu(c) ? nullptr : Dinv,
                                              c->imp.rhs + k * 5 * nc, S.b + k * S.ldv, red);
   if (S.packed) {
-    enqueue_pack(s, (int)nc, A, 0, 5, S.A16 + k * packed_words(nc, 5));
-    if (!uses_ilu(c)) enqueue_pack(s, (int)nc, Dinv, 0, 1, S.D16 + k * packed_words(nc, 1));
+    enqueue_pack(s, (int)nc, A, 5, 0, 5, S.A16 + k * packed_words(nc, 5));
+    if (!uses_ilu(c)) enqueue_pack(s, (int)nc, Dinv, 1, 0, 1, S.D16 + k * packed_words(nc, 1));
   }
   reduce_rows_kernel<<<15, 256, 0, s>>>(red, nb, 10, 1, norms);
   stamp(c, s, PROF_ASSEMBLE, 0);
@@ -588,7 +588,7 @@ void enqueue_factor(const Sys<T, B>& S, cudaStream_t s, int k) {
   T* Dinv = S.Dinv_of(k);
   stamp(c, s, PROF_ILU_FACTOR, 1);
   copy_vec_kernel<T><<<dim3(kRedBlocks, 1), 256, 0, s>>>(slots(LU, 0), cslots((const T*)S.A_of(k), 0),
-                                                        125 * nc, nullptr);
+                                                        block_values(nc, 5), nullptr);
   for (int q = 0; q < M.n_stages; ++q) {
     const int n = M.stage_off[q + 1] - M.stage_off[q];
     if (c->imp.use_colour_ranges) {
@@ -604,8 +604,8 @@ void enqueue_factor(const Sys<T, B>& S, cudaStream_t s, int k) {
     }
   }
   if (S.packed) {
-    enqueue_pack(s, (int)nc, LU, 1, 4, S.LU16 + k * packed_words(nc, 4));
-    enqueue_pack(s, (int)nc, Dinv, 0, 1, S.D16 + k * packed_words(nc, 1));
+    enqueue_pack(s, (int)nc, LU, 5, 1, 4, S.LU16 + k * packed_words(nc, 4));
+    enqueue_pack(s, (int)nc, Dinv, 1, 0, 1, S.D16 + k * packed_words(nc, 1));
   }
   stamp(c, s, PROF_ILU_FACTOR, 0);
 }
@@ -623,11 +623,11 @@ int reset_grid_sync(bes_ctx* c) {
 
 // The linear solves as one persistent launch (gmres_persistent.cuh) or as the graph's kernels:
 // persistent while the rows between two waits (a colour, or all of them with block Jacobi) are
-// no more than a few times what the grid's warps hold at six rows each.  A step's solve, graph
-// against persistent, measured (ms, one step at CFL 50): block ILU 7k cells FP32 4.5 / 2.2, 20k
-// FP64 9.0 / 4.8, 74k packed 7.8 / 5.9, FP32 10.5 / 6.6, FP64 20.5 / 14.9, 5 x 20k packed 8.2 / 6.3,
-// 150k FP32 23.5 / 15.1; 150k packed 11.5 / 14.5 (2.2 times: its sweeps are the fast ones of the
-// graph).  Block Jacobi: 20k FP64 12.2 / 8.6, 74k FP32 11.2 / 8.8 (5.1 times).
+// no more than a few times what the grid's warps hold at six rows each.  Two steps at CFL 50, graph
+// against persistent, measured in ms with the multiple in brackets: block ILU FP32 12k cells 7.5 /
+// 5.0, 52k 12.1 / 7.4, 74k (1.0) 13.7 / 12.5, 130k (1.8) 19.2 / 19.8; FP64 12k 13.3 / 7.0, 52k (1.4)
+// 21.5 / 20.2, 74k (2.0) 25.9 / 27.9; packed 12k 7.8 / 5.3, 74k (1.0) 13.5 / 10.9.  Block Jacobi: FP64
+// 33k (4.5) 29.3 / 22.5, FP32 74k (5.1) 21.1 / 16.2.
 void choose_solve(bes_ctx* c) {
   ImplicitBuffers& I = c->imp;
   I.solve_blocks = 0;
@@ -642,7 +642,7 @@ void choose_solve(bes_ctx* c) {
   }
   const int64_t blocks = std::min<int64_t>(I.solve_resident, (rows + 31) / 32);
   const double held = (double)kRowsPerWarp * 8 * blocks;
-  if (stage > held * (!uses_ilu(c) ? 5.5 : (I.packed ? 1.75 : 2.5))) return;
+  if (stage > held * (uses_ilu(c) ? 1.6 : 5.5)) return;
   I.solve_lane_spmv = rows <= 1.25 * held;
   if (uses_ilu(c) && !I.Y && imp_malloc(c, &I.Y, I.ldv * I.tsize * I.nslot)) return;
   I.solve_blocks = (int)blocks;
@@ -1144,12 +1144,12 @@ int implicit_allocate(bes_ctx* c) {
   I.ldv = basis_stride(nc);
   // the system in T: per condition, or one scratch shared by all (16-bit storage)
   const int64_t msl = I.packed ? 1 : ns;
-  I.sA = I.packed ? 0 : 125 * nc;
-  I.sDinv = I.packed ? 0 : 25 * nc;
+  I.sA = I.packed ? 0 : block_values(nc, 5);
+  I.sDinv = I.packed ? 0 : block_values(nc, 1);
   int rc = 0;
-  rc |= imp_malloc(c, &I.A, 125 * nc * I.tsize * msl);
-  rc |= imp_malloc(c, &I.Dinv, 25 * nc * I.tsize * msl);
-  if (uses_ilu(c)) rc |= imp_malloc(c, &I.LU, 125 * nc * I.tsize * msl);
+  rc |= imp_malloc(c, &I.A, block_values(nc, 5) * I.tsize * msl);
+  rc |= imp_malloc(c, &I.Dinv, block_values(nc, 1) * I.tsize * msl);
+  if (uses_ilu(c)) rc |= imp_malloc(c, &I.LU, block_values(nc, 5) * I.tsize * msl);
   if (I.packed) {
     rc |= imp_malloc(c, (void**)&I.A16, packed_words(nc, 5) * sizeof(uint32_t) * ns);
     rc |= imp_malloc(c, (void**)&I.D16, packed_words(nc, 1) * sizeof(uint32_t) * ns);
@@ -1191,7 +1191,7 @@ int implicit_allocate(bes_ctx* c) {
   rc |= imp_malloc(c, (void**)&I.stage_rows, nc * sizeof(int32_t));
   rc |= imp_malloc(c, (void**)&I.ilu_pos, nc * sizeof(int32_t));
   if (rc) return BES_ERR_CUDA;
-  IMP_TRY(c, cudaMemset(I.A, 0, 125 * nc * I.tsize * msl));  // empty slots stay zero
+  IMP_TRY(c, cudaMemset(I.A, 0, block_values(nc, 5) * I.tsize * msl));  // empty slots stay zero
   IMP_TRY(c, cudaMemset(g.lin, 0, ns * sizeof(int32_t)));
   IMP_TRY(c, cudaMemset(g.cyc, 0, ns * sizeof(int32_t)));
   IMP_TRY(c, cudaMemset(g.counters, 0, 3 * sizeof(unsigned long long)));
@@ -1324,9 +1324,9 @@ int bes_implicit_assemble(bes_ctx* ctx, double cfl, double* rhs, double* blocks,
       for (int v = 0; v < 5; ++v) rhs[M.cell_new2ref[i] * 5 + v] = h[v * nc + i];
   }
   if (blocks) {
-    std::vector<double> A(125 * nc);
+    std::vector<double> A(block_values(nc, 5));
     if (ctx->imp.prec) {
-      std::vector<float> Af(125 * nc);
+      std::vector<float> Af(A.size());
       IMP_TRY(ctx, cudaMemcpy(Af.data(), ctx->imp.A, Af.size() * sizeof(float), cudaMemcpyDeviceToHost));
       for (size_t k = 0; k < Af.size(); ++k) A[k] = Af[k];
     } else {
@@ -1339,7 +1339,8 @@ int bes_implicit_assemble(bes_ctx* ctx, double cfl, double* rhs, double* blocks,
       const int64_t i = M.cell_ref2new[c];
       for (int s = 0; s < 5; ++s) {
         if (s > 0 && R.cadj[c * 4 + (s - 1)] < 0) continue;
-        for (int q = 0; q < 25; ++q) blocks[k * 25 + q] = A[(size_t)(s * 25 + q) * nc + i];
+        for (int q = 0; q < 25; ++q)
+          blocks[k * 25 + q] = A[ctx->imp.prec ? block_at<float>(5, s, q, i) : block_at<double>(5, s, q, i)];
         ++k;
       }
     }

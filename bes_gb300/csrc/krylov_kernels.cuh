@@ -69,6 +69,11 @@ __device__ __forceinline__ float ld_once(const float* a, uint64_t pol) {
   asm("ld.global.nc.L2::cache_hint.f32 %0, [%1], %2;" : "=f"(v) : "l"(a), "l"(pol));
   return v;
 }
+__device__ __forceinline__ double ld_once(const double* a, uint64_t pol) {
+  double v;
+  asm("ld.global.nc.L2::cache_hint.f64 %0, [%1], %2;" : "=d"(v) : "l"(a), "l"(pol));
+  return v;
+}
 __device__ __forceinline__ uint4 ld_once(const uint4* a, uint64_t pol) {
   uint4 v;
   asm("ld.global.nc.L2::cache_hint.v4.u32 {%0, %1, %2, %3}, [%4], %5;"
@@ -85,6 +90,21 @@ __device__ __forceinline__ PackedBlock load_packed_once(const uint32_t* __restri
   for (int p = 0; p < 3; ++p) b.q[p] = ld_once(reinterpret_cast<const uint4*>(w + packed_word(4 * p, i)), pol);
   b.last = ld_once(w + packed_word(12, i), pol);
   return b;
+}
+
+// load_block with the evict_first policy
+template <class T>
+__device__ __forceinline__ void load_block_once(const T* A, int nslots, int s, int i, T* a, uint64_t pol) {
+  constexpr int W = Vec16<T>::W;
+  const uint4* p = reinterpret_cast<const uint4*>(A + block_at<T>(nslots, s, 0, i));
+#pragma unroll
+  for (int k = 0; k < 24 / W; ++k) {
+    const uint4 u = ld_once(p + k * 32, pol);
+    const T* v = reinterpret_cast<const T*>(&u);
+#pragma unroll
+    for (int e = 0; e < W; ++e) a[k * W + e] = v[e];
+  }
+  a[24] = ld_once(A + block_at<T>(nslots, s, 24, i), pol);
 }
 
 // ---- gathers of a cell's five values ------------------------------------------------------------
@@ -134,6 +154,11 @@ __device__ __forceinline__ void gather5(const double* __restrict__ x, int j, dou
 __device__ __forceinline__ float fma_t(float a, float b, float c) { return fmaf(a, b, c); }
 __device__ __forceinline__ double fma_t(double a, double b, double c) { return fma(a, b, c); }
 
+// Resident blocks of 128 threads that the row kernels of an unpacked system are compiled for (their
+// registers hold a whole block).
+template <class T>
+constexpr int kRowBlocks = sizeof(T) == 4 ? 8 : 5;
+
 // ---- preconditioners ------------------------------------------------------------------------
 
 // Colour-ordered block-ILU(0) sweep when the colours are contiguous cell ranges in increasing
@@ -151,29 +176,37 @@ __device__ __forceinline__ void ilu_colour_row(const DevMesh& m, int i, int r0, 
                                                const T* __restrict__ Dinv,
                                                const T* __restrict__ in, T* __restrict__ out) {
   const int nc = m.nc;
+  const uint64_t pol = l2_evict_first();
   const T* own = (LOWER || r0 == 0) ? in : out;
+  // the four neighbour ids first (one round trip), then the qualifying slots
+  int jn[4];
+#pragma unroll
+  for (int s = 0; s < 4; ++s) jn[s] = m.adj[s * nc + i];
   T acc[5];
   gather5<COH>(own, i, acc);
 #pragma unroll
   for (int s = 0; s < 4; ++s) {
-    const int j = m.adj[s * nc + i];
+    const int j = jn[s];
     const bool lower = LOWER && j >= 0 && j < r0;
     const bool upper = UPPER && j >= r1;
     if (!lower && !upper) continue;
     const T* src = (lower && j < s1) ? in : out;
-    T y[5];
+    T y[5], a[25];
+    load_block_once(A, 5, 1 + s, i, a, pol);
     gather5<COH>(src, j, y);
 #pragma unroll
     for (int r = 0; r < 5; ++r)
 #pragma unroll
-      for (int c = 0; c < 5; ++c) acc[r] = fma_t(-ellc(A, 1 + s, r * 5 + c, nc, i), y[c], acc[r]);
+      for (int c = 0; c < 5; ++c) acc[r] = fma_t(-a[r * 5 + c], y[c], acc[r]);
   }
   if (UPPER) {
+    T a[25];
+    load_block_once(Dinv, 1, 0, i, a, pol);
 #pragma unroll
     for (int r = 0; r < 5; ++r) {
       T x = T(0);
 #pragma unroll
-      for (int c = 0; c < 5; ++c) x = fma_t(Dinv[(int64_t)(r * 5 + c) * nc + i], acc[c], x);
+      for (int c = 0; c < 5; ++c) x = fma_t(a[r * 5 + c], acc[c], x);
       out[(int64_t)i * 5 + r] = x;
     }
   } else {
@@ -183,7 +216,7 @@ __device__ __forceinline__ void ilu_colour_row(const DevMesh& m, int i, int r0, 
 }
 
 template <class T, bool LOWER, bool UPPER, bool BATCH>
-__global__ void __launch_bounds__(128) ilu_colour_kernel(DevMesh m, int r0, int r1, int s1,
+__global__ void __launch_bounds__(128, kRowBlocks<T>) ilu_colour_kernel(DevMesh m, int r0, int r1, int s1,
                                                          SlotPtr<const T> Ap, SlotPtr<const T> Dp,
                                                          SlotPtr<const T> inp, SlotPtr<T> outp,
                                                          const int32_t* run) {
@@ -464,13 +497,14 @@ __global__ void __launch_bounds__(128) ilu_lower_kernel(DevMesh m, const int32_t
   for (int s = 0; s < 4; ++s) {
     const int j = m.adj[s * nc + i];
     if (j < 0 || pos[j] >= pi) continue;
-    T y[5];
+    T y[5], a[25];
+    load_block(A, 5, 1 + s, i, a);
 #pragma unroll
     for (int v = 0; v < 5; ++v) y[v] = z[(int64_t)j * 5 + v];
 #pragma unroll
     for (int r = 0; r < 5; ++r)
 #pragma unroll
-      for (int c = 0; c < 5; ++c) acc[r] -= ellc(A, 1 + s, r * 5 + c, nc, i) * y[c];
+      for (int c = 0; c < 5; ++c) acc[r] = fma_t(-a[r * 5 + c], y[c], acc[r]);
   }
 #pragma unroll
   for (int v = 0; v < 5; ++v) z[(int64_t)i * 5 + v] = acc[v];
@@ -497,19 +531,22 @@ __global__ void __launch_bounds__(128) ilu_upper_kernel(DevMesh m, const int32_t
   for (int s = 0; s < 4; ++s) {
     const int k = m.adj[s * nc + i];
     if (k < 0 || pos[k] <= pi) continue;
-    T y[5];
+    T y[5], a[25];
+    load_block(A, 5, 1 + s, i, a);
 #pragma unroll
     for (int v = 0; v < 5; ++v) y[v] = z[(int64_t)k * 5 + v];
 #pragma unroll
     for (int r = 0; r < 5; ++r)
 #pragma unroll
-      for (int c = 0; c < 5; ++c) acc[r] -= ellc(A, 1 + s, r * 5 + c, nc, i) * y[c];
+      for (int c = 0; c < 5; ++c) acc[r] = fma_t(-a[r * 5 + c], y[c], acc[r]);
   }
+  T d[25];
+  load_block(Dinv, 1, 0, i, d);
 #pragma unroll
   for (int r = 0; r < 5; ++r) {
     T x = T(0);
 #pragma unroll
-    for (int c = 0; c < 5; ++c) x += Dinv[(int64_t)(r * 5 + c) * nc + i] * acc[c];
+    for (int c = 0; c < 5; ++c) x = fma_t(d[r * 5 + c], acc[c], x);
     z[(int64_t)i * 5 + r] = x;
   }
 }
@@ -528,15 +565,15 @@ __global__ void __launch_bounds__(256) copy_vec_kernel(SlotPtr<T> outp, SlotPtr<
 
 // block-Jacobi application: out_i = Dinv_i in_i
 template <class T, bool COH>
-__device__ __forceinline__ void jacobi_row(int nc, int i, const T* __restrict__ Dinv, const T* in,
-                                           T* out) {
-  T x[5];
+__device__ __forceinline__ void jacobi_row(int i, const T* __restrict__ Dinv, const T* in, T* out) {
+  T x[5], a[25];
+  load_block_once(Dinv, 1, 0, i, a, l2_evict_first());
   gather5<COH>(in, i, x);
 #pragma unroll
   for (int r = 0; r < 5; ++r) {
     T acc = T(0);
 #pragma unroll
-    for (int c = 0; c < 5; ++c) acc += Dinv[(int64_t)(r * 5 + c) * nc + i] * x[c];
+    for (int c = 0; c < 5; ++c) acc = fma_t(a[r * 5 + c], x[c], acc);
     out[(int64_t)i * 5 + r] = acc;
   }
 }
@@ -546,7 +583,7 @@ __global__ void __launch_bounds__(256) jacobi_apply_kernel(int nc, SlotPtr<const
                                                            const int32_t* run) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= nc || slot_idle(run)) return;
-  jacobi_row<T, false>(nc, i, Dp.at(), inp.at(), outp.at());
+  jacobi_row<T, false>(i, Dp.at(), inp.at(), outp.at());
 }
 
 // block-Jacobi application with a packed inverse diagonal
@@ -575,38 +612,37 @@ static __global__ void __launch_bounds__(256) jacobi_apply_packed_kernel(
 
 // ---- matrix-vector products ------------------------------------------------------------------
 
-// Row i of y = A x (ELL), or y = b - A x when b is given
+// Row i of y = A x, or y = b - A x when b is given
 template <class T, bool COH>
 __device__ __forceinline__ void spmv_row(const DevMesh& m, int i, const T* __restrict__ A,
                                          const T* x, const T* __restrict__ b, T* y) {
   const int nc = m.nc;
-  T acc[5], xi[5];
-  gather5<COH>(x, i, xi);
+  const uint64_t pol = l2_evict_first();
+  int jn[5];
+  jn[0] = i;
 #pragma unroll
-  for (int r = 0; r < 5; ++r) {
-    T s = T(0);
+  for (int s = 1; s < 5; ++s) jn[s] = m.adj[(s - 1) * nc + i];
+  T acc[5] = {T(0), T(0), T(0), T(0), T(0)};
 #pragma unroll
-    for (int c = 0; c < 5; ++c) s += ellc(A, 0, r * 5 + c, nc, i) * xi[c];
-    acc[r] = s;
-  }
-#pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    const int j = m.adj[q * nc + i];
-    if (j < 0) continue;
-    gather5<COH>(x, j, xi);
+  for (int s = 0; s < 5; ++s) {
+    if (jn[s] < 0) continue;
+    T xs[5], a[25];
+    load_block_once(A, 5, s, i, a, pol);
+    gather5<COH>(x, jn[s], xs);
 #pragma unroll
     for (int r = 0; r < 5; ++r)
 #pragma unroll
-      for (int c = 0; c < 5; ++c) acc[r] += ellc(A, 1 + q, r * 5 + c, nc, i) * xi[c];
+      for (int c = 0; c < 5; ++c) acc[r] = fma_t(a[r * 5 + c], xs[c], acc[r]);
   }
 #pragma unroll
   for (int r = 0; r < 5; ++r)
     y[(int64_t)i * 5 + r] = b ? b[(int64_t)i * 5 + r] - acc[r] : acc[r];
 }
 template <class T, bool BATCH>
-__global__ void __launch_bounds__(256) spmv_kernel(DevMesh m, SlotPtr<const T> Ap,
-                                                   SlotPtr<const T> xp, SlotPtr<const T> bp,
-                                                   SlotPtr<T> yp, const int32_t* run) {
+__global__ void __launch_bounds__(128, kRowBlocks<T>) spmv_kernel(DevMesh m, SlotPtr<const T> Ap,
+                                                                  SlotPtr<const T> xp,
+                                                                  SlotPtr<const T> bp, SlotPtr<T> yp,
+                                                                  const int32_t* run) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= m.nc || slot_idle(run)) return;
   spmv_row<T, false>(m, i, sat<BATCH>(Ap), sat<BATCH>(xp), bp.p ? sat<BATCH>(bp) : nullptr,
@@ -651,7 +687,7 @@ __device__ __forceinline__ void spmv_packed_row(const DevMesh& m, int i, const u
 // Blocks of 128 with 12 of them resident: more loads in flight than the registers of a row that
 // the compiler would keep (2.16M cells: 129 us without the bound, 102 with 12 or 8, 125 with 16).
 template <bool BATCH>
-__global__ void __launch_bounds__(128, 12) spmv_packed_kernel(
+__global__ void __launch_bounds__(128, BATCH ? 10 : 12) spmv_packed_kernel(
     DevMesh m, SlotPtr<const uint32_t> Hp, SlotPtr<const float> xp, SlotPtr<const float> bp,
     SlotPtr<float> yp, const int32_t* run) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
