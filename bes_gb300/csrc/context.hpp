@@ -125,10 +125,10 @@ struct ImplicitBuffers {
   // 0/1) or one shared scratch (precision 2); sA etc. are the per-condition strides in elements
   // (0: shared)
   void* A = nullptr;
-  void* LU = nullptr;    // block-ILU(0) factors in the same layout (ILU only)
+  void* LU = nullptr;    // block-ILU(0) factors in the same layout (ILU only; precision 2: A itself)
   void* Dinv = nullptr;  // 1 slot: inverse diagonal (Jacobi) / inverse U_ii (ILU)
   int64_t sA = 0, sDinv = 0;
-  void* Dc = nullptr;    // per-face diagonal contributions [2][25][nf] (shared)
+  void* Jf = nullptr;    // per-face flux derivatives, 2 slots by groups of 32 faces (shared)
   // Krylov side, per condition
   void* b = nullptr;     // right-hand side in T [ldv]
   void* V = nullptr;     // Krylov basis [(m+1)][ldv] (FP16 with precision 2)

@@ -66,7 +66,7 @@ struct Sys {
   bes_ctx* c;
   int nc, nslot;
   int64_t N, ldv, sV, sA, sDinv;
-  T *A, *LU, *Dinv, *Dc, *b, *Z, *W, *X, *Vx;
+  T *A, *LU, *Dinv, *Jf, *b, *Z, *W, *X, *Vx;
   B* V;
   bool packed, basis16;
   uint32_t *A16, *LU16, *D16;
@@ -85,7 +85,7 @@ struct Sys {
     A = (T*)I.A;
     LU = (T*)I.LU;
     Dinv = (T*)I.Dinv;
-    Dc = (T*)I.Dc;
+    Jf = (T*)I.Jf;
     b = (T*)I.b;
     Z = (T*)I.Z;
     W = (T*)I.W;
@@ -530,14 +530,6 @@ void enqueue_residual_all(bes_ctx* c, cudaStream_t s, const SlotHandles& hs, int
   stamp(c, s, PROF_RESIDUAL, 0);
 }
 
-// 16-bit block-scaled copies (precision 2; T is float there)
-template <class T>
-void enqueue_pack(cudaStream_t s, int nc, const T* src, int src_slots, int slot0, int nslots,
-                  uint32_t* H) {
-  if constexpr (std::is_same<T, float>::value)
-    pack_blocks_kernel<<<dim3(nblk(nc, 256), nslots), 256, 0, s>>>(src, src_slots, slot0, nc, H);
-}
-
 // Slot k: first-order Jacobians, the assembled system with its right-hand side, the 16-bit
 // copies (precision 2) and the step's norms (into norms [15]: L2 of the right-hand side [5],
 // L2 of R [5], max of the right-hand side [5]).
@@ -554,30 +546,33 @@ void enqueue_assembly(const Sys<T, B>& S, cudaStream_t s, int k, double* norms) 
   Params prm = c->prm;
   prm.pinf_dev = c->pinf_dev + 6 * k;
   prm.active = nullptr;
-  FaceLocal fl{c->imp.m_own, c->imp.m_nb};
-  T* A = S.A_of(k);
-  T* Dinv = S.Dinv_of(k);
+  const FaceLocal fl{c->imp.m_own, c->imp.m_nb};
+  // the factorisation works on a second copy, or (16-bit storage) on A itself
+  AssembleOut<T> out;
+  std::memset(&out, 0, sizeof(out));
+  out.A = S.A_of(k);
+  if (uses_ilu(c) && !S.packed) out.LU = S.LU_of(k);
+  if (!uses_ilu(c)) out.Dinv = S.Dinv_of(k);
+  if (S.packed) {
+    out.A16 = S.A16 + k * packed_words(nc, 5);
+    out.D16 = S.D16 + k * packed_words(nc, 1);
+  }
   double* red = c->imp.red + (int64_t)k * 64 * c->imp.red_ld;
   stamp(c, s, PROF_JACOBIAN, 1);
-  face_jacobian_kernel<T><<<nblk(nf, 128), 128, 0, s>>>(m, prm, fl, U, dt, dtmin, local,
-                                                        o.jacobian_repeat, A, S.Dc);
+  face_jacobian_kernel<T><<<nblk(nf, 128), 128, 0, s>>>(m, prm, U, S.Jf);
   stamp(c, s, PROF_JACOBIAN, 0);
   stamp(c, s, PROF_ASSEMBLE, 1);
   const int nb = nblk(nc, 128);
-  cell_assemble_kernel<T><<<nb, 128, 0, s>>>(m, c->FA + k * kFaW * nf, dt, dtmin, local,
-                                             o.jacobian_repeat, S.Dc, A,
-                                             uses_ilu(c) ? nullptr : Dinv,
+  cell_assemble_kernel<T><<<nb, 128, 0, s>>>(m, fl, c->FA + k * kFaW * nf, dt, dtmin, local,
+                                             o.jacobian_repeat, S.Jf, out,
                                              c->imp.rhs + k * 5 * nc, S.b + k * S.ldv, red);
-  if (S.packed) {
-    enqueue_pack(s, (int)nc, A, 5, 0, 5, S.A16 + k * packed_words(nc, 5));
-    if (!uses_ilu(c)) enqueue_pack(s, (int)nc, Dinv, 1, 0, 1, S.D16 + k * packed_words(nc, 1));
-  }
   reduce_rows_kernel<<<15, 256, 0, s>>>(red, nb, 10, 1, norms);
   stamp(c, s, PROF_ASSEMBLE, 0);
 }
 
-// Slot k: block-ILU(0) factorisation of a copy of A, stage by stage (the factorisation of the
-// stage's rows, then the inverses of their diagonal blocks), and its 16-bit copies.
+// Slot k: block-ILU(0) factorisation in place in LU (which the assembly wrote), stage by stage: the
+// factorisation of the stage's rows, then the inverses of their diagonal blocks and their 16-bit
+// copies.
 template <class T, class B>
 void enqueue_factor(const Sys<T, B>& S, cudaStream_t s, int k) {
   bes_ctx* c = S.c;
@@ -586,26 +581,21 @@ void enqueue_factor(const Sys<T, B>& S, cudaStream_t s, int k) {
   const int64_t nc = S.nc;
   T* LU = S.LU_of(k);
   T* Dinv = S.Dinv_of(k);
+  uint32_t* LU16 = S.packed ? S.LU16 + k * packed_words(nc, 4) : nullptr;
+  uint32_t* D16 = S.packed ? S.D16 + k * packed_words(nc, 1) : nullptr;
   stamp(c, s, PROF_ILU_FACTOR, 1);
-  copy_vec_kernel<T><<<dim3(kRedBlocks, 1), 256, 0, s>>>(slots(LU, 0), cslots((const T*)S.A_of(k), 0),
-                                                        block_values(nc, 5), nullptr);
   for (int q = 0; q < M.n_stages; ++q) {
     const int n = M.stage_off[q + 1] - M.stage_off[q];
+    const int32_t* rows = c->imp.stage_rows + M.stage_off[q];
     if (c->imp.use_colour_ranges) {
       ilu_factor_kernel<T, true><<<nblk(n, 128), 128, 0, s>>>(c->dm, nullptr, n, nullptr, LU, Dinv,
                                                               M.stage_off[q]);
-      ilu_invert_kernel<T, true><<<nblk(n, 128), 128, 0, s>>>(c->dm, nullptr, n, LU, Dinv,
+      ilu_invert_kernel<T, true><<<nblk(n, 128), 128, 0, s>>>(c->dm, nullptr, n, LU, Dinv, LU16, D16,
                                                               M.stage_off[q]);
     } else {
-      ilu_factor_kernel<T><<<nblk(n, 128), 128, 0, s>>>(c->dm, c->imp.stage_rows + M.stage_off[q],
-                                                        n, c->imp.ilu_pos, LU, Dinv);
-      ilu_invert_kernel<T><<<nblk(n, 128), 128, 0, s>>>(c->dm, c->imp.stage_rows + M.stage_off[q],
-                                                        n, LU, Dinv);
+      ilu_factor_kernel<T><<<nblk(n, 128), 128, 0, s>>>(c->dm, rows, n, c->imp.ilu_pos, LU, Dinv);
+      ilu_invert_kernel<T><<<nblk(n, 128), 128, 0, s>>>(c->dm, rows, n, LU, Dinv, LU16, D16);
     }
-  }
-  if (S.packed) {
-    enqueue_pack(s, (int)nc, LU, 5, 1, 4, S.LU16 + k * packed_words(nc, 4));
-    enqueue_pack(s, (int)nc, Dinv, 1, 0, 1, S.D16 + k * packed_words(nc, 1));
   }
   stamp(c, s, PROF_ILU_FACTOR, 0);
 }
@@ -1149,13 +1139,14 @@ int implicit_allocate(bes_ctx* c) {
   int rc = 0;
   rc |= imp_malloc(c, &I.A, block_values(nc, 5) * I.tsize * msl);
   rc |= imp_malloc(c, &I.Dinv, block_values(nc, 1) * I.tsize * msl);
-  if (uses_ilu(c)) rc |= imp_malloc(c, &I.LU, block_values(nc, 5) * I.tsize * msl);
+  if (uses_ilu(c) && !I.packed) rc |= imp_malloc(c, &I.LU, block_values(nc, 5) * I.tsize * msl);
+  if (I.packed) I.LU = I.A;
   if (I.packed) {
     rc |= imp_malloc(c, (void**)&I.A16, packed_words(nc, 5) * sizeof(uint32_t) * ns);
     rc |= imp_malloc(c, (void**)&I.D16, packed_words(nc, 1) * sizeof(uint32_t) * ns);
     if (uses_ilu(c)) rc |= imp_malloc(c, (void**)&I.LU16, packed_words(nc, 4) * sizeof(uint32_t) * ns);
   }
-  rc |= imp_malloc(c, &I.Dc, 50 * nf * I.tsize);
+  rc |= imp_malloc(c, &I.Jf, block_values(nf, 2) * I.tsize);
   rc |= imp_malloc(c, &I.b, I.ldv * I.tsize * ns);
   I.sV = (int64_t)(o.gmres_restart + 1) * I.ldv;
   rc |= imp_malloc(c, &I.V, I.sV * (I.basis16 ? sizeof(__half) : I.tsize) * ns);
@@ -1192,6 +1183,7 @@ int implicit_allocate(bes_ctx* c) {
   rc |= imp_malloc(c, (void**)&I.ilu_pos, nc * sizeof(int32_t));
   if (rc) return BES_ERR_CUDA;
   IMP_TRY(c, cudaMemset(I.A, 0, block_values(nc, 5) * I.tsize * msl));  // empty slots stay zero
+  if (I.packed) IMP_TRY(c, cudaMemset(I.A16, 0, packed_words(nc, 5) * sizeof(uint32_t) * ns));
   IMP_TRY(c, cudaMemset(g.lin, 0, ns * sizeof(int32_t)));
   IMP_TRY(c, cudaMemset(g.cyc, 0, ns * sizeof(int32_t)));
   IMP_TRY(c, cudaMemset(g.counters, 0, 3 * sizeof(unsigned long long)));

@@ -16,6 +16,7 @@
 #include <type_traits>
 
 #include "explicit_kernels.cuh"
+#include "flux_jacobian.cuh"
 
 namespace bes {
 
@@ -68,6 +69,90 @@ __device__ __forceinline__ void store_block(T* A, int nslots, int s, int i, cons
     *reinterpret_cast<uint4*>(p + k * 32 * W) = u;
   }
   A[block_at<T>(nslots, s, 24, i)] = a[24];
+}
+
+// ---- 16-bit block-scaled storage of the FP32 system (precision 2)
+// Entry q of a 5x5 block = scale * half q.  The scale is the smallest power of two >= the block's
+// largest |entry|, so the rescaling is exact and every stored entry lies in [-1, 1] with FP16's
+// 11-bit significand; entries below 2^-14 of the scale become FP16 subnormals (absolute error at
+// most 2^-25 of the scale).  A block is 13 words: words 0..11 the halves 0..23, word 12 the
+// half 24 and, in its upper 16 bits, the upper 16 bits of the FP32 scale (a power of two has no
+// others).  52 bytes instead of 100.
+// Layout: groups of 32 rows; within a group slot after slot; of a slot first words 0..3 of the 32
+// rows, then words 4..7, words 8..11 (16 bytes per row each) and words 12.  A warp reads a block
+// with three 16-byte loads and one of 4 bytes per lane, and its group's slots are one contiguous
+// piece.  With one 4-byte array per word and a separate scale (14 loads and streams per block) an
+// application on 2.16M cells took 194 us and a product 147 us, now 147 and 102.
+constexpr int kBlockWords = 13;
+constexpr int kGroupWords = 32 * kBlockWords;
+inline int64_t packed_words(int64_t nc, int nslots) { return (nc + 31) / 32 * nslots * kGroupWords; }
+// the words of slot s of row i's group
+__device__ __forceinline__ const uint32_t* packed_slot(const uint32_t* H, int nslots, int s, int i) {
+  return H + ((int64_t)(i >> 5) * nslots + s) * kGroupWords;
+}
+// word p of row i within its slot
+__device__ __forceinline__ int packed_word(int p, int i) {
+  return p < 12 ? (p >> 2) * 128 + (i & 31) * 4 + (p & 3) : 384 + (i & 31);
+}
+__device__ __forceinline__ float packed_scale(uint32_t last) {
+  return __uint_as_float(last & 0xffff0000u);
+}
+struct PackedBlock {
+  uint4 q[3];
+  uint32_t last;
+  // the entries (without the scale); returns the scale
+  __device__ __forceinline__ float unpack(float* a) const {
+    const uint32_t w[kBlockWords] = {q[0].x, q[0].y, q[0].z, q[0].w, q[1].x, q[1].y, q[1].z,
+                                     q[1].w, q[2].x, q[2].y, q[2].z, q[2].w, last};
+#pragma unroll
+    for (int p = 0; p < 12; ++p) {
+      const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w[p]));
+      a[2 * p] = f.x;
+      a[2 * p + 1] = f.y;
+    }
+    a[24] = __low2float(*reinterpret_cast<const __half2*>(&w[12]));
+    return packed_scale(last);
+  }
+};
+
+// smallest power of two >= x (x >= 0 and finite); 1 for x == 0
+__device__ __forceinline__ float pow2_ceil(float x) {
+  if (x == 0.0f) return 1.0f;
+  const unsigned b = __float_as_uint(x);
+  return __uint_as_float((b + 0x007fffffu) & 0xff800000u);
+}
+
+// a (row-major block) into slot s of row i
+__device__ __forceinline__ void store_packed(uint32_t* __restrict__ H, int nslots, int s, int i,
+                                             const float* a) {
+  float mx = 0.0f;
+#pragma unroll
+  for (int q = 0; q < 25; ++q) mx = fmaxf(mx, fabsf(a[q]));
+  const float sc = pow2_ceil(mx);
+  const float inv = 1.0f / sc;  // exact: sc is a power of two
+  uint32_t w[12];
+#pragma unroll
+  for (int p = 0; p < 12; ++p) {
+    const __half2 h = __floats2half2_rn(a[2 * p] * inv, a[2 * p + 1] * inv);
+    w[p] = *reinterpret_cast<const uint32_t*>(&h);
+  }
+  uint32_t* base = H + ((int64_t)(i >> 5) * nslots + s) * kGroupWords;
+#pragma unroll
+  for (int p = 0; p < 3; ++p)
+    *reinterpret_cast<uint4*>(base + packed_word(4 * p, i)) =
+        make_uint4(w[4 * p], w[4 * p + 1], w[4 * p + 2], w[4 * p + 3]);
+  base[packed_word(12, i)] =
+      (uint32_t)__half_as_ushort(__float2half_rn(a[24] * inv)) | (__float_as_uint(sc) & 0xffff0000u);
+}
+
+// block of slot s of row i
+__device__ __forceinline__ PackedBlock load_packed(const uint32_t* __restrict__ H, int nslots, int s, int i) {
+  const uint32_t* w = packed_slot(H, nslots, s, i);
+  PackedBlock b;
+#pragma unroll
+  for (int p = 0; p < 3; ++p) b.q[p] = *reinterpret_cast<const uint4*>(w + packed_word(4 * p, i));
+  b.last = w[packed_word(12, i)];
+  return b;
 }
 
 // a[k] for a runtime k in [0, 4) without indexing the array (keeps it in registers)
@@ -127,22 +212,16 @@ __device__ __forceinline__ void inv5(const T* a, T* inv) {
 // ---------------------------------------------------------------------------------------
 // Jacobians and assembly (SolverImplicit::computeFaceFluxes_, src/SolverImplicit.cpp:358-507)
 // ---------------------------------------------------------------------------------------
-struct FaceLocal {
-  const int8_t* m_own;  // local face index of the face in its owner
-  const int8_t* m_nb;   // ... in its neighbour (-1 on boundary faces)
-};
-
-// Per face: dF/dU_L and dF/dU_R at the FIRST-order states (the two cell averages) by
-// forward-mode derivatives of the flux templates (two passes of 5 slots).  Writes the
-// face's two off-diagonal blocks (each added `rep` times from zero, as the reference's
-// addToBlock sits inside the variable loop, quirk Q9) and its contributions to the two
-// diagonal blocks (m_o J_L for the owner, -m_n J_R for the neighbour) for the cell sweep.
+// Per face: dF/dU_L (slot 0) and, for interior faces, dF/dU_R (slot 1) at the FIRST-order states (the
+// two cell averages), in the block layout by groups of 32 faces.  A warp writes whole sectors; the
+// cells read both blocks of their faces and scale them.  Written per face into the cells' rows
+// (scattered blocks and the diagonals' contributions, twice the bytes) and differentiated with
+// all five derivatives of every quantity, this took 2.8 ms on 2.16M cells (FP32) and 5.4 ms on
+// 518,400 (FP64, bound by the FP64 pipe), now 0.7 and 2.5.
 template <class T>
-__global__ void __launch_bounds__(128) face_jacobian_kernel(
-    DevMesh m, Params prm, FaceLocal fl, const double* __restrict__ U,
-    const double* __restrict__ dt, const unsigned long long* __restrict__ dtmin, int local_dt,
-    int rep, T* __restrict__ A, T* __restrict__ Dc) {
-  typedef Dual<5, T> DT;
+__global__ void __launch_bounds__(128) face_jacobian_kernel(DevMesh m, Params prm,
+                                                            const double* __restrict__ U,
+                                                            T* __restrict__ Jf) {
   const int f = blockIdx.x * blockDim.x + threadIdx.x;
   const int nc = m.nc, nf = m.nf;
   if (f >= nf) return;
@@ -150,21 +229,28 @@ __global__ void __launch_bounds__(128) face_jacobian_kernel(
   double n[3];
 #pragma unroll
   for (int d = 0; d < 3; ++d) n[d] = m.fn[(int64_t)d * nf + f];
-  const double area = m.farea[f];
-  const double dtg = local_dt ? 0.0 : __longlong_as_double((long long)*dtmin);
-  const double m_o = (local_dt ? dt[o] : dtg) * m.inv_vol[o] * area;
-  T JL[25], JR[25];
   T ul[5], ur[5];
 #pragma unroll
   for (int v = 0; v < 5; ++v) ul[v] = (T)U[(int64_t)v * nc + o];
   const bool interior = f < m.nf_int;
-  int nb = -1;
   if (interior) {
-    nb = m.fnb[f];
+    const int nb = m.fnb[f];
 #pragma unroll
     for (int v = 0; v < 5; ++v) ur[v] = (T)U[(int64_t)v * nc + nb];
   }
-  GasConst g = prm.gas;
+  const GasConst g = prm.gas;
+  if constexpr (std::is_same<T, double>::value) {
+    if (interior) {
+      T J[25];
+      roe_derivative<T>(g, var_side<T>(g, ul, n), fixed_side<T>(g, ur, n), n, J);
+      store_block(Jf, 2, 0, f, J);
+      roe_derivative<T>(g, fixed_side<T>(g, ul, n), var_side<T>(g, ur, n), n, J);
+      store_block(Jf, 2, 1, f, J);
+      return;
+    }
+  }
+  typedef Dual<5, T> DT;
+  T JL[25], JR[25];
   for (int side = 0; side < (interior ? 2 : 1); ++side) {
     DT dl[5], dr[5], dfl[5];
 #pragma unroll
@@ -184,45 +270,58 @@ __global__ void __launch_bounds__(128) face_jacobian_kernel(
       freestream_flux(g, dl, prm.pinf_dev, n, dfl);
     T* J = side == 0 ? JL : JR;
 #pragma unroll
-    for (int a = 0; a < 5; ++a)
+    for (int r = 0; r < 5; ++r)
 #pragma unroll
-      for (int b = 0; b < 5; ++b) J[a * 5 + b] = dfl[a].d[b];
+      for (int c = 0; c < 5; ++c) J[r * 5 + c] = dfl[r].d[c];
   }
-  const T mo = (T)m_o;
-#pragma unroll
-  for (int q = 0; q < 25; ++q) Dc[(int64_t)q * nf + f] = mo * JL[q];
-  if (interior) {
-    const double m_n = (local_dt ? dt[nb] : dtg) * m.inv_vol[nb] * area;
-    const T mn = (T)m_n;
-    const int so = 1 + fl.m_own[f], sn = 1 + fl.m_nb[f];
-    T bo[25], bn[25];
-#pragma unroll
-    for (int q = 0; q < 25; ++q) {
-      Dc[(int64_t)(25 + q) * nf + f] = -mn * JR[q];
-      const T yo = mo * JR[q], yn = -mn * JL[q];
-      T xo = T(0), xn = T(0);
-      for (int r = 0; r < rep; ++r) {
-        xo += yo;
-        xn += yn;
-      }
-      bo[q] = xo;
-      bn[q] = xn;
-    }
-    store_block(A, 5, so, o, bo);
-    store_block(A, 5, sn, nb, bn);
-  }
+  store_block(Jf, 2, 0, f, JL);
+  if (interior) store_block(Jf, 2, 1, f, JR);
 }
 
+// D += m J, `rep` times.  FP32: each product rounded once and added `rep` times, in the order in
+// which the system was always formed.  FP64: rep m J with one rounding (the additions would
+// take a thousand FP64 instructions per cell).
+__device__ __forceinline__ void add_scaled(float* J, float m, int rep, float* D) {
+#pragma unroll
+  for (int q = 0; q < 25; ++q) J[q] = __fmul_rn(m, J[q]);
+#pragma unroll 1
+  for (int r = 0; r < rep; ++r)
+#pragma unroll
+    for (int q = 0; q < 25; ++q) D[q] += J[q];
+}
+__device__ __forceinline__ void add_scaled(const double* J, double m, int rep, double* D) {
+  const double k = (double)rep * m;
+#pragma unroll
+  for (int q = 0; q < 25; ++q) D[q] = fma(k, J[q], D[q]);
+}
+
+struct FaceLocal {
+  const int8_t* m_own;  // local face index of the face in its owner
+  const int8_t* m_nb;   // ... in its neighbour (-1 on boundary faces)
+};
+
+// Outputs of the assembly; null where a context has no use for one.
+template <class T>
+struct AssembleOut {
+  T* A;
+  T* LU;          // a second copy, for the factorisation
+  T* Dinv;        // inverse diagonal (block Jacobi)
+  uint32_t* A16;  // packed A and inverse diagonal
+  uint32_t* D16;
+};
+
 // Per cell: right-hand side -(dt/V) sum(+-F A) in the reference's face order, the diagonal
-// block I + rep * sum of the face contributions, block-Jacobi inverse (optional), and block
-// partial norms of the right-hand side.
+// block I + rep * sum of the face contributions (m J_L of the faces it owns, -m J_R of the others,
+// m = dt / V * area), the off-diagonal blocks (m J_R, -m J_L, each added `rep` times from zero, as
+// the reference's addToBlock sits inside the variable loop, quirk Q9), block-Jacobi inverse
+// (optional), and block partial norms of the right-hand side.
 template <class T>
 __global__ void __launch_bounds__(128) cell_assemble_kernel(
-    DevMesh m, const double* __restrict__ FA, const double* __restrict__ dt,
-    const unsigned long long* __restrict__ dtmin, int local_dt, int rep, const T* __restrict__ Dc,
-    T* __restrict__ A, T* __restrict__ Dinv, double* __restrict__ rhs, T* __restrict__ rhs_t,
+    DevMesh m, FaceLocal fl, const double* __restrict__ FA, const double* __restrict__ dt,
+    const unsigned long long* __restrict__ dtmin, int local_dt, int rep, const T* __restrict__ Jf,
+    AssembleOut<T> out, double* __restrict__ rhs, T* __restrict__ rhs_t,
     double* __restrict__ partials) {
-  const int nc = m.nc, nf = m.nf;
+  const int nc = m.nc;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   double b[5] = {0, 0, 0, 0, 0};
   double R[5] = {0, 0, 0, 0, 0};  // unscaled residual sum(+-F A), for convergence monitoring
@@ -232,31 +331,46 @@ __global__ void __launch_bounds__(128) cell_assemble_kernel(
     T D[25];
 #pragma unroll
     for (int q = 0; q < 25; ++q) D[q] = (q % 6 == 0) ? T(1) : T(0);
-#pragma unroll
+#pragma unroll 1
     for (int s = 0; s < 4; ++s) {
       const int gf = m.gface[s * nc + i];
       if (gf == bes::kNoFace) continue;  // empty slot of a triangle
-      const int f = gf >= 0 ? gf : ~gf;
+      const bool own = gf >= 0;
+      const int f = own ? gf : ~gf;
       double fa[5];
       load_fa(FA, f, fa);
 #pragma unroll
       for (int v = 0; v < 5; ++v) {
-        const double x = k * fa[v];
-        b[v] = gf >= 0 ? b[v] - x : b[v] + x;
-        R[v] = gf >= 0 ? R[v] + fa[v] : R[v] - fa[v];
+        const double y = k * fa[v];
+        b[v] = own ? b[v] - y : b[v] + y;
+        R[v] = own ? R[v] + fa[v] : R[v] - fa[v];
       }
-      const T* src = Dc + (gf >= 0 ? 0 : (int64_t)25 * nf);
+      const T mf = (T)(k * m.farea[f]), sm = own ? mf : -mf;
+      T J[25];
+      load_block(Jf, 2, own ? 0 : 1, f, J);
+      add_scaled(J, sm, rep, D);
+      if (f >= m.nf_int) continue;
+      load_block(Jf, 2, own ? 1 : 0, f, J);
+      T x[25];
 #pragma unroll
-      for (int q = 0; q < 25; ++q) {
-        const T y = src[(int64_t)q * nf + f];
-        for (int r = 0; r < rep; ++r) D[q] += y;
-      }
+      for (int q = 0; q < 25; ++q) x[q] = T(0);
+      add_scaled(J, sm, rep, x);
+      const int slot = 1 + (own ? fl.m_own[f] : fl.m_nb[f]);
+      store_block(out.A, 5, slot, i, x);
+      if (out.LU) store_block(out.LU, 5, slot, i, x);
+      if constexpr (std::is_same<T, float>::value)
+        if (out.A16) store_packed(out.A16, 5, slot, i, x);
     }
-    store_block(A, 5, 0, i, D);
-    if (Dinv) {
+    store_block(out.A, 5, 0, i, D);
+    if (out.LU) store_block(out.LU, 5, 0, i, D);
+    if constexpr (std::is_same<T, float>::value)
+      if (out.A16) store_packed(out.A16, 5, 0, i, D);
+    if (out.Dinv) {
       T inv[25];
       inv5(D, inv);
-      store_block(Dinv, 1, 0, i, inv);
+      store_block(out.Dinv, 1, 0, i, inv);
+      if constexpr (std::is_same<T, float>::value)
+        if (out.D16) store_packed(out.D16, 1, 0, i, inv);
     }
 #pragma unroll
     for (int v = 0; v < 5; ++v) {
@@ -401,110 +515,29 @@ __global__ void __launch_bounds__(128) ilu_factor_kernel(DevMesh m, const int32_
   }
 }
 
-// inverse of the factored diagonal block of each row of a stage (after ilu_factor_kernel)
+// inverse of the factored diagonal block of each row of a stage (after ilu_factor_kernel), and
+// the row's packed copies (LU16, D16; null without them)
 template <class T, bool RANGE = false>
 __global__ void __launch_bounds__(128) ilu_invert_kernel(DevMesh m, const int32_t* __restrict__ rows,
                                                          int nrows, const T* __restrict__ A,
-                                                         T* __restrict__ Dinv, int r0 = 0) {
+                                                         T* __restrict__ Dinv, uint32_t* __restrict__ LU16,
+                                                         uint32_t* __restrict__ D16, int r0 = 0) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= nrows) return;
-  const int nc = m.nc;
   const int i = RANGE ? r0 + t : rows[t];
   T D[25], inv[25];
   load_block(A, 5, 0, i, D);
   inv5(D, inv);
   store_block(Dinv, 1, 0, i, inv);
-}
-
-// ---- 16-bit block-scaled storage of the FP32 system (precision 2)
-// Entry q of a 5x5 block = scale * half q.  The scale is the smallest power of two >= the block's
-// largest |entry|, so the rescaling is exact and every stored entry lies in [-1, 1] with FP16's
-// 11-bit significand; entries below 2^-14 of the scale become FP16 subnormals (absolute error at
-// most 2^-25 of the scale).  A block is 13 words: words 0..11 the halves 0..23, word 12 the
-// half 24 and, in its upper 16 bits, the upper 16 bits of the FP32 scale (a power of two has no
-// others).  52 bytes instead of 100.
-// Layout: groups of 32 rows; within a group slot after slot; of a slot first words 0..3 of the 32
-// rows, then words 4..7, words 8..11 (16 bytes per row each) and words 12.  A warp reads a block
-// with three 16-byte loads and one of 4 bytes per lane, and its group's slots are one contiguous
-// piece.  With one 4-byte array per word and a separate scale (14 loads and streams per block) an
-// application on 2.16M cells took 194 us and a product 147 us, now 147 and 102.
-constexpr int kBlockWords = 13;
-constexpr int kGroupWords = 32 * kBlockWords;
-inline int64_t packed_words(int64_t nc, int nslots) { return (nc + 31) / 32 * nslots * kGroupWords; }
-// the words of slot s of row i's group
-__device__ __forceinline__ const uint32_t* packed_slot(const uint32_t* H, int nslots, int s, int i) {
-  return H + ((int64_t)(i >> 5) * nslots + s) * kGroupWords;
-}
-// word p of row i within its slot
-__device__ __forceinline__ int packed_word(int p, int i) {
-  return p < 12 ? (p >> 2) * 128 + (i & 31) * 4 + (p & 3) : 384 + (i & 31);
-}
-__device__ __forceinline__ float packed_scale(uint32_t last) {
-  return __uint_as_float(last & 0xffff0000u);
-}
-struct PackedBlock {
-  uint4 q[3];
-  uint32_t last;
-  // the entries (without the scale); returns the scale
-  __device__ __forceinline__ float unpack(float* a) const {
-    const uint32_t w[kBlockWords] = {q[0].x, q[0].y, q[0].z, q[0].w, q[1].x, q[1].y, q[1].z,
-                                     q[1].w, q[2].x, q[2].y, q[2].z, q[2].w, last};
-#pragma unroll
-    for (int p = 0; p < 12; ++p) {
-      const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w[p]));
-      a[2 * p] = f.x;
-      a[2 * p + 1] = f.y;
+  if constexpr (std::is_same<T, float>::value)
+    if (LU16) {
+      store_packed(D16, 1, 0, i, inv);
+#pragma unroll 1
+      for (int s = 0; s < 4; ++s) {
+        load_block(A, 5, 1 + s, i, D);
+        store_packed(LU16, 4, s, i, D);
+      }
     }
-    a[24] = __low2float(*reinterpret_cast<const __half2*>(&w[12]));
-    return packed_scale(last);
-  }
-};
-
-// smallest power of two >= x (x >= 0 and finite); 1 for x == 0
-__device__ __forceinline__ float pow2_ceil(float x) {
-  if (x == 0.0f) return 1.0f;
-  const unsigned b = __float_as_uint(x);
-  return __uint_as_float((b + 0x007fffffu) & 0xff800000u);
-}
-
-// pack slots [slot0, slot0 + gridDim.y) of A (nslots slots) into H's gridDim.y slots; one thread
-// per (cell, slot)
-static __global__ void __launch_bounds__(256) pack_blocks_kernel(const float* __restrict__ A, int nslots,
-                                                                 int slot0, int nc,
-                                                                 uint32_t* __restrict__ H) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  const int s = blockIdx.y;
-  if (i >= nc) return;
-  float a[25];
-  float mx = 0.0f;
-  load_block(A, nslots, slot0 + s, i, a);
-#pragma unroll
-  for (int q = 0; q < 25; ++q) mx = fmaxf(mx, fabsf(a[q]));
-  const float sc = pow2_ceil(mx);
-  const float inv = 1.0f / sc;  // exact: sc is a power of two
-  uint32_t w[12];
-#pragma unroll
-  for (int p = 0; p < 12; ++p) {
-    const __half2 h = __floats2half2_rn(a[2 * p] * inv, a[2 * p + 1] * inv);
-    w[p] = *reinterpret_cast<const uint32_t*>(&h);
-  }
-  uint32_t* base = H + ((int64_t)(i >> 5) * gridDim.y + s) * kGroupWords;
-#pragma unroll
-  for (int p = 0; p < 3; ++p)
-    *reinterpret_cast<uint4*>(base + packed_word(4 * p, i)) =
-        make_uint4(w[4 * p], w[4 * p + 1], w[4 * p + 2], w[4 * p + 3]);
-  base[packed_word(12, i)] =
-      (uint32_t)__half_as_ushort(__float2half_rn(a[24] * inv)) | (__float_as_uint(sc) & 0xffff0000u);
-}
-
-// block of slot s of row i
-__device__ __forceinline__ PackedBlock load_packed(const uint32_t* __restrict__ H, int nslots, int s, int i) {
-  const uint32_t* w = packed_slot(H, nslots, s, i);
-  PackedBlock b;
-#pragma unroll
-  for (int p = 0; p < 3; ++p) b.q[p] = *reinterpret_cast<const uint4*>(w + packed_word(4 * p, i));
-  b.last = w[packed_word(12, i)];
-  return b;
 }
 
 }  // namespace bes
