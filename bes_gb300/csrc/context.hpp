@@ -152,6 +152,7 @@ struct ImplicitBuffers {
   GmresDev gm;
   StepResult* res = nullptr;   // [slot]
   std::vector<StepResult> res_host;
+  unsigned* gs_done = nullptr;  // [slot] finished rows of the Gram-Schmidt sums
   double* cfl_dev = nullptr;   // [slot] CFL of the current step
   int32_t* act = nullptr;      // [slot] slots that take the current step
   int32_t* guard_dev = nullptr;  // restart-cycle limit of a linear solve (device copy)

@@ -756,7 +756,7 @@ __device__ __noinline__ void phase_reduce(const SolveArgs<T, B>& S, int rows, in
   }
 }
 
-// |w|^2 - |h|^2 of a slot (gs_decide_kernel's sum, in order), the same in every lane of the warp.
+// |w|^2 - |h|^2 of a slot (gs_decide's sum, in order), the same in every lane of the warp.
 __device__ __forceinline__ double decide_norm2(const double* dev, int nv) {
   const int lane = threadIdx.x & 31;
   const double h = lane < nv ? __ldcg(dev + lane) : 0.0;
@@ -767,51 +767,6 @@ __device__ __forceinline__ double decide_norm2(const double* dev, int nv) {
     s = fma(d, d, s);
   }
   return nw2 - s;
-}
-
-// gmres_givens_kernel for one slot by one warp: the rotations' products that do not depend on
-// the carried entry are taken by all lanes at once, which leaves one multiplication and one
-// addition per rotation in series.
-__device__ __noinline__ void givens_warp(const GmresDev& g, const GmresParam& P, int t, int j) {
-  const int lane = threadIdx.x & 31;
-  double* H = g.H + (int64_t)t * kHsize;
-  double* cs = g.cs + (int64_t)t * kMaxRestart;
-  double* sn = g.sn + (int64_t)t * kMaxRestart;
-  double* gg = g.g + (int64_t)t * (kMaxRestart + 1);
-  const double* dev = g.dev + (int64_t)t * kGsLd;
-  const bool second = __ldcg(dev + kGsFlag) != 0.0;
-  // lane i: entry i of the new column, rotation i
-  double h = 0.0, c = 0.0, s = 0.0;
-  if (lane <= j) h = second ? __dadd_rn(__ldcg(dev + lane), __ldcg(dev + kGsH2 + lane)) : __ldcg(dev + lane);
-  if (lane < j) {
-    c = __ldcg(cs + lane);
-    s = __ldcg(sn + lane);
-  }
-  const double below = __shfl_down_sync(0xffffffffu, h, 1);  // entry lane + 1 before its rotation
-  const double sb = __dmul_rn(s, below), cb = __dmul_rn(c, below);
-  double a = __shfl_sync(0xffffffffu, h, 0), mine = a;
-  for (int i = 0; i < j; ++i) {
-    if (lane == i) mine = a;
-    a = __dadd_rn(__dmul_rn(-__shfl_sync(0xffffffffu, s, i), a), __shfl_sync(0xffffffffu, cb, i));
-  }
-  if (lane < j) H[lane * kHld + j] = __dadd_rn(__dmul_rn(c, mine), sb);
-  if (lane == 0) {
-    const double hn = __ldcg(dev + kGsNorm);
-    const double d = sqrt(__dadd_rn(__dmul_rn(a, a), __dmul_rn(hn, hn)));
-    const double cj = d == 0.0 ? 1.0 : a / d, sj = d == 0.0 ? 0.0 : hn / d;
-    cs[j] = cj;
-    sn[j] = sj;
-    H[j * kHld + j] = d;
-    H[(j + 1) * kHld + j] = 0.0;
-    const double gj = __ldcg(gg + j), gn = __dmul_rn(-sj, gj);
-    gg[j + 1] = gn;
-    gg[j] = __dmul_rn(cj, gj);
-    g.jc[t] = j + 1;
-    const int it = __ldcg(g.iter + t) + 1;
-    g.iter[t] = it;
-    if (second) g.second[t] = __ldcg(g.second + t) + 1;
-    g.cyc[t] = (!(fabs(gn) <= __ldcg(g.sc + 8 * t + 1)) && j + 1 < P.mr && it < P.maxiter) ? 1 : 0;
-  }
 }
 
 // y = H^{-1} g of one slot by one warp (gmres_solve_y_kernel): a row's products at once, then
@@ -935,7 +890,7 @@ __global__ void __launch_bounds__(256, std::is_same<T, double>::value ? 1 : 2) g
       if (!bar()) return;
       phase_reduce(S, nv + 1, nvb_g, 0, run_sh, nullptr);
       if (!bar()) return;
-      // gs_decide_kernel stage 1, by every block, a warp per slot
+      // gs_decide stage 1, by every block, a warp per slot
       int re = 0;
       for (int k = tid >> 5; k < ns; k += 8) {
         if (!run_sh[k]) continue;
@@ -969,7 +924,7 @@ __global__ void __launch_bounds__(256, std::is_same<T, double>::value ? 1 : 2) g
         if (!bar()) return;
         phase_reduce(S, nv + 1, nvb_g, kGsH2, run_sh, second_sh);
         if (!bar()) return;
-        // gs_decide_kernel stage 2
+        // gs_decide_kernel
         for (int k = tid >> 5; k < ns; k += 8) {
           if (!run_sh[k] || second_sh[k] != 1) continue;
           double* dev = g.dev + (int64_t)k * kGsLd;

@@ -431,32 +431,36 @@ int enqueue_arnoldi(const Sys<T, B>& S, cudaStream_t s, int j, const GmresParam&
   stamp(c, s, PROF_SPMV, 0);
   stamp(c, s, PROF_ORTHO, 1);
   const auto Vb = S.cbasis(0);
+  GsOut out;
+  out.dev = S.dev();
+  out.devf = S.devf();
+  out.done = c->imp.gs_done;
+  out.second = h.gs2[j];
+  out.set_second = h.on;
+  const GivensArgs ga{c->imp.gm, P, h, S.nslot, j};
   launch_gs_dots<T, B>(nv, S.vgrid, s, Vb, S.ldv, S.cvec(S.W), S.N, S.red(), cyc);
-  reduce_slots_kernel<<<dim3(nv + 1, S.nslot), 256, 0, s>>>(S.cred(), kRedBlocks, nv + 1, 0,
-                                                            S.dev(), cyc);
-  gs_decide_kernel<<<dim3(1, S.nslot), 64, 0, s>>>(S.dev(), S.devf(), nv, 1, cyc, h.gs2[j],
-                                                    h.on, nullptr);
+  gs_sums_kernel<<<dim3(nv + 1, S.nslot), 256, 0, s>>>(S.cred(), out, cyc);
   launch_gs_update<T, B, GS_FINAL1>(nv, S.vgrid, s, S.basis(j + 1), S.vec(S.Vx), S.vec(S.W), Vb,
-                                    S.ldv, S.cdev(), S.cdevf(), S.N, S.red(), cyc);
+                                    S.ldv, S.cdev(), S.cdevf(), S.N, S.red(), cyc, ga);
   // the second pass (rare): in the step graph an IF node that runs only when a slot needs it,
-  // so that its four launches cost nothing otherwise
+  // so that its launches cost nothing otherwise
   cudaStream_t s2 = s;
   if (h.on) {
     s2 = c->imp.cap[2];
     if (const int rc = begin_conditional(c, s, s2, h.gs2[j], cudaGraphCondTypeIf)) return rc;
   }
   launch_gs_update<T, B, GS_REORTH>(nv, S.vgrid, s2, S.basis(j + 1), S.vec(S.Vx), S.vec(S.W), Vb,
-                                    S.ldv, S.cdev(), S.cdevf(), S.N, S.red(), cyc);
+                                    S.ldv, S.cdev(), S.cdevf(), S.N, S.red(), cyc, ga);
   reduce_slots_kernel<<<dim3(nv + 1, S.nslot), 256, 0, s2>>>(S.cred(), kRedBlocks, nv + 1, 0,
                                                              S.dev(kGsH2), cyc);
-  gs_decide_kernel<<<dim3(1, S.nslot), 64, 0, s2>>>(S.dev(), S.devf(), nv, 2, cyc, h.gs2[j],
-                                                     h.on, h.on ? c->imp.gm.counters + 2 : nullptr);
+  gs_decide_kernel<<<dim3(1, S.nslot), 64, 0, s2>>>(S.dev(), S.devf(), nv, cyc, h.gs2[j], h.on,
+                                                     h.on ? c->imp.gm.counters + 2 : nullptr);
   launch_gs_update<T, B, GS_FINAL2>(nv, S.vgrid, s2, S.basis(j + 1), S.vec(S.Vx), S.vec(S.W), Vb,
-                                    S.ldv, S.cdev(), S.cdevf(), S.N, S.red(), cyc);
+                                    S.ldv, S.cdev(), S.cdevf(), S.N, S.red(), cyc, ga);
+  gmres_givens_kernel<<<1, 256, 0, s2>>>(ga);
   if (h.on) {
     if (const int rc = end_conditional(c, s2, gs2_kernels)) return rc;
   }
-  gmres_givens_kernel<<<1, S.nthr, 0, s>>>(c->imp.gm, P, h, S.nslot, j);
   stamp(c, s, PROF_ORTHO, 0);
   return BES_OK;
 }
@@ -1174,6 +1178,7 @@ int implicit_allocate(bes_ctx* c) {
   rc |= imp_malloc(c, (void**)&I.act, ns * sizeof(int32_t));
   rc |= imp_malloc(c, (void**)&I.guard_dev, sizeof(int32_t));
   rc |= imp_malloc(c, (void**)&c->prof.dev, 3 * PROF_NCAT * sizeof(unsigned long long));
+  rc |= imp_malloc(c, (void**)&I.gs_done, ns * sizeof(unsigned));
   rc |= imp_malloc(c, (void**)&I.sync_count, sizeof(unsigned));
   rc |= imp_malloc(c, (void**)&I.sync_gen, sizeof(unsigned));
   rc |= imp_malloc(c, (void**)&I.sync_error, sizeof(int));
@@ -1188,6 +1193,7 @@ int implicit_allocate(bes_ctx* c) {
   IMP_TRY(c, cudaMemset(g.cyc, 0, ns * sizeof(int32_t)));
   IMP_TRY(c, cudaMemset(g.counters, 0, 3 * sizeof(unsigned long long)));
   IMP_TRY(c, cudaMemset(I.guard_dev, 0, sizeof(int32_t)));
+  IMP_TRY(c, cudaMemset(I.gs_done, 0, ns * sizeof(unsigned)));
   IMP_TRY(c, cudaMemset(I.sync_count, 0, sizeof(unsigned)));
   IMP_TRY(c, cudaMemset(I.sync_gen, 0, sizeof(unsigned)));
   IMP_TRY(c, cudaMemset(I.sync_error, 0, sizeof(int)));

@@ -803,20 +803,24 @@ static __global__ void __launch_bounds__(256) reduce_slots_kernel(
 // states the same algorithm):
 //   pass 1   h = V^T w and |w|^2 in one read of V and w (gs_dots_kernel);
 //   decide   |w - V h|^2 = |w|^2 - |h|^2 (Pythagoras); a second pass runs only when this
-//            is <= kReorthTheta2 |w|^2 (gs_decide_kernel, on the device);
+//            is <= kReorthTheta2 |w|^2 (gs_sums_kernel, its block that finishes last);
 //   no second pass: V_{j+1} = (w - V h) / sqrt(|w|^2 - |h|^2) in one more read of V and w
-//            (gs_update_kernel<FINAL1>);
+//            (gs_update_kernel<FINAL1>, with the Givens update of the step in one more block);
 //   second pass: w -= V h with V^T w and |w|^2 of the result in the same read
 //            (gs_update_kernel<REORTH>), then V_{j+1} = (w - V h2) / norm (<FINAL2>).
 // The kernels of the path not taken return at once.  Device scalars per slot (dev):
 //   dev[0..nv-1] h, dev[nv] |w|^2; dev[kGsH2 + k] h2, dev[kGsH2 + nv] |w'|^2;
 //   dev[kGsFlag] 1 if the second pass runs, dev[kGsInv] 1/h_{j+1,j} (0: leave V_{j+1}),
-//   dev[kGsNorm] h_{j+1,j}; dev[kGsR] a vector's squared norm (start and restart).
-//   devf: FP32 copies of h, h2, the flag and 1/h_{j+1,j} at the same offsets, written by
-//   gs_decide_kernel, so that FP32 update kernels convert nothing per thread.
+//   dev[kGsNorm] h_{j+1,j}; dev[kGsR] a vector's squared norm (start and restart);
+//   dev[kGsOn] 1 if the slot takes the step (the Givens update clears its run flag meanwhile).
+//   devf: FP32 copies of h, h2, the flags and 1/h_{j+1,j} at the same offsets, so that FP32
+//   update kernels convert nothing per thread.
+// With the decision and the Givens update in launches of their own, the latter one thread per slot,
+// the step's Gram-Schmidt took 49.7 us on four conditions of 81,000 cells and 160 us on 2.16M cells
+// (16-bit storage), now 38.8 and 142.
 constexpr double kReorthTheta2 = 1.0 / 16.0;
-constexpr int kGsH2 = 40, kGsFlag = 80, kGsInv = 81, kGsNorm = 82, kGsR = 83;
-static_assert(kGsR < kGsLd, "Gram-Schmidt scalars per slot");
+constexpr int kGsH2 = 40, kGsFlag = 80, kGsInv = 81, kGsNorm = 82, kGsR = 83, kGsOn = 84;
+static_assert(kGsOn < kGsLd, "Gram-Schmidt scalars per slot");
 
 template <class A>
 __device__ __forceinline__ const A* gs_coef(const double* dev, const float* devf);
@@ -915,6 +919,173 @@ struct BasisIO<float, __half> {
   }
 };
 
+struct GmresParam {
+  int mr;         // restart length
+  int maxiter;    // linear iteration limit
+  double tol;     // relative tolerance
+};
+
+struct GmresHandles {
+  cudaGraphConditionalHandle loop;              // WHILE over restart cycles
+  cudaGraphConditionalHandle arn[kMaxRestart];  // IF of Arnoldi step j
+  cudaGraphConditionalHandle gs2[kMaxRestart];  // IF of step j's second Gram-Schmidt pass
+  int on;                                       // 0: not inside a conditional graph
+};
+
+constexpr int kHsize = (kMaxRestart + 1) * kHld;  // Hessenberg entries per slot
+
+__device__ __forceinline__ void set_arnoldi_handles(const GmresHandles& h, int from, int mr,
+                                                    unsigned first) {
+  if (!h.on) return;
+  for (int k = from; k < mr; ++k) cudaGraphSetConditional(h.arn[k], k == from ? first : 0u);
+}
+
+// A slot's stage-1 decision (one block; h and |w|^2 in tot[0..nv]): the second-pass flag and,
+// without a second pass, 1/h_{j+1,j}.  Inside the step graph the second pass is the body of an IF
+// node on `second` (set_second != 0).
+__device__ __forceinline__ void gs_decide(const double* tot, int nv, double* dev, float* devf,
+                                          cudaGraphConditionalHandle second, int set_second) {
+  for (int k = threadIdx.x; k < nv; k += blockDim.x) devf[k] = (float)tot[k];
+  if (threadIdx.x != 0) return;
+  const double nw2 = tot[nv];
+  double s = 0.0;
+  for (int k = 0; k < nv; ++k) s = fma(tot[k], tot[k], s);
+  const double est = nw2 - s;
+  const bool reorth = !(est > kReorthTheta2 * nw2);
+  if (reorth && set_second) cudaGraphSetConditional(second, 1u);
+  const double hn = reorth ? 0.0 : sqrt(est), inv = hn > 0.0 ? 1.0 / hn : 0.0;
+  dev[kGsFlag] = reorth ? 1.0 : 0.0;
+  dev[kGsNorm] = hn;
+  dev[kGsInv] = inv;
+  dev[kGsOn] = 1.0;
+  devf[kGsFlag] = reorth ? 1.0f : 0.0f;
+  devf[kGsInv] = (float)inv;
+  devf[kGsOn] = 1.0f;
+}
+
+// Sums of the nv + 1 rows of partials (a block per row, grid (nv + 1, slots), the trees of
+// reduce_slots_kernel) into dev; the slot's last block decides.  (The last block of the dots itself
+// would take 7 us for the sums of 13 rows: FP64 additions of a single SM.)
+struct GsOut {
+  SlotPtr<double> dev;
+  SlotPtr<float> devf;
+  unsigned* done;  // [slot] finished rows, 0 between launches
+  cudaGraphConditionalHandle second;
+  int set_second;
+};
+static __global__ void __launch_bounds__(256) gs_sums_kernel(SlotPtr<const double> pp, GsOut out,
+                                                             const int32_t* run) {
+  double* dev = out.dev.at();
+  float* devf = out.devf.at();
+  if (slot_idle(run)) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+      dev[kGsOn] = 0.0;
+      devf[kGsOn] = 0.0f;
+    }
+    return;
+  }
+  __shared__ double sh[8], tot[kMaxRestart + 1];
+  __shared__ int last;
+  const double* row = pp.at() + (int64_t)blockIdx.x * kRedBlocks;
+  double x = 0.0;
+#pragma unroll
+  for (int b = 0; b < kRedBlocks; b += 256) x += row[b + threadIdx.x];
+  x = warp_sum(x);
+  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = x;
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    x = warp_sum(threadIdx.x < 8 ? sh[threadIdx.x] : 0.0);
+    if (threadIdx.x == 0) {
+      dev[blockIdx.x] = x;
+      __threadfence();
+      last = atomicAdd(out.done + blockIdx.y, 1u) == gridDim.x - 1;
+      if (last) out.done[blockIdx.y] = 0;
+      __threadfence();
+    }
+  }
+  __syncthreads();
+  if (!last) return;
+  const int nv = gridDim.x - 1;
+  if (threadIdx.x <= nv) tot[threadIdx.x] = __ldcg(dev + threadIdx.x);
+  __syncthreads();
+  gs_decide(tot, nv, dev, devf, out.second, out.set_second);
+}
+
+// Arnoldi step j of one slot, by one warp: column j of the Hessenberg matrix from the slot's
+// coefficients, the earlier Givens rotations applied to it, a new rotation that zeroes h_{j+1,j},
+// and the rotated right-hand side; the slot's cycle stops when |g_{j+1}| <= eps, at the restart
+// length, or at the iteration limit.  Rotation arithmetic without FMA contraction; the rotations'
+// products that do not depend on the carried entry are taken by all lanes at once, which leaves one
+// multiplication and one addition per rotation in series.
+__device__ __noinline__ void givens_warp(const GmresDev& g, const GmresParam& P, int t, int j) {
+  const int lane = threadIdx.x & 31;
+  double* H = g.H + (int64_t)t * kHsize;
+  double* cs = g.cs + (int64_t)t * kMaxRestart;
+  double* sn = g.sn + (int64_t)t * kMaxRestart;
+  double* gg = g.g + (int64_t)t * (kMaxRestart + 1);
+  const double* dev = g.dev + (int64_t)t * kGsLd;
+  const bool second = __ldcg(dev + kGsFlag) != 0.0;
+  // lane i: entry i of the new column, rotation i
+  double h = 0.0, c = 0.0, s = 0.0;
+  if (lane <= j) h = second ? __dadd_rn(__ldcg(dev + lane), __ldcg(dev + kGsH2 + lane)) : __ldcg(dev + lane);
+  if (lane < j) {
+    c = __ldcg(cs + lane);
+    s = __ldcg(sn + lane);
+  }
+  const double below = __shfl_down_sync(0xffffffffu, h, 1);  // entry lane + 1 before its rotation
+  const double sb = __dmul_rn(s, below), cb = __dmul_rn(c, below);
+  double a = __shfl_sync(0xffffffffu, h, 0), mine = a;
+  for (int i = 0; i < j; ++i) {
+    if (lane == i) mine = a;
+    a = __dadd_rn(__dmul_rn(-__shfl_sync(0xffffffffu, s, i), a), __shfl_sync(0xffffffffu, cb, i));
+  }
+  if (lane < j) H[lane * kHld + j] = __dadd_rn(__dmul_rn(c, mine), sb);
+  if (lane == 0) {
+    const double hn = __ldcg(dev + kGsNorm);
+    const double d = sqrt(__dadd_rn(__dmul_rn(a, a), __dmul_rn(hn, hn)));
+    const double cj = d == 0.0 ? 1.0 : a / d, sj = d == 0.0 ? 0.0 : hn / d;
+    cs[j] = cj;
+    sn[j] = sj;
+    H[j * kHld + j] = d;
+    H[(j + 1) * kHld + j] = 0.0;
+    const double gj = __ldcg(gg + j), gn = __dmul_rn(-sj, gj);
+    gg[j + 1] = gn;
+    gg[j] = __dmul_rn(cj, gj);
+    g.jc[t] = j + 1;
+    const int it = __ldcg(g.iter + t) + 1;
+    g.iter[t] = it;
+    if (second) g.second[t] = __ldcg(g.second + t) + 1;
+    g.cyc[t] = (!(fabs(gn) <= __ldcg(g.sc + 8 * t + 1)) && j + 1 < P.mr && it < P.maxiter) ? 1 : 0;
+  }
+}
+
+// The Givens updates of Arnoldi step j by one block, for the slots that run the step with
+// (pass = 1) or without (0) a second Gram-Schmidt pass, and the condition of the next step: a
+// slot whose second pass is still to come counts as running.
+struct GivensArgs {
+  GmresDev g;
+  GmresParam P;
+  GmresHandles h;
+  int nslot, j;
+};
+__device__ __forceinline__ void givens_block(const GivensArgs& a, int pass) {
+  for (int t = threadIdx.x >> 5; t < a.nslot; t += blockDim.x >> 5)
+    if (__ldcg(a.g.cyc + t) && (__ldcg(a.g.dev + (int64_t)t * kGsLd + kGsFlag) != 0.0) == (pass != 0))
+      givens_warp(a.g, a.P, t, a.j);
+  __threadfence_block();
+  __syncthreads();
+  int cont = 0;
+  for (int t = threadIdx.x; t < a.nslot; t += blockDim.x) cont |= __ldcg(a.g.cyc + t);
+  const int any = __syncthreads_or(cont);
+  if (threadIdx.x != 0) return;
+  if (pass == 0) ++a.g.counters[0];
+  if (a.j + 1 < a.P.mr) set_arnoldi_handles(a.h, a.j + 1, a.P.mr, any ? 1u : 0u);
+}
+// ... after the second pass
+static __global__ void __launch_bounds__(256) gmres_givens_kernel(const __grid_constant__ GivensArgs a) {
+  givens_block(a, 1);
+}
+
 // Pass 1: partial V_k . w (rows k < NV) and |w|^2 (row NV).
 template <class T, class B, int NV>
 __global__ void __launch_bounds__(256) gs_dots_kernel(SlotPtr<const B> Vp, int64_t ldv,
@@ -963,17 +1134,13 @@ __global__ void __launch_bounds__(256) gs_dots_kernel(SlotPtr<const B> Vp, int64
   block_reduce_store<NV + 1, A>(acc, pp.at());
 }
 
-// Decide after a reduction (grid (1, slots)): stage 1 (after pass 1) sets the second-pass
-// flag and, without a second pass, 1/h_{j+1,j}; stage 2 (after pass 2) sets 1/h_{j+1,j} from
-// the second pass.  Inside the step graph the second pass is the body of an IF node on
-// `second` (set_second != 0): stage 1 sets it to 1 for a slot that needs the pass, and stage 2,
-// which runs inside that body, sets it back to 0 for the next Arnoldi step of this index and
-// counts the body's executions in *passes.
+// Decide after the second pass (grid (1, slots)): 1/h_{j+1,j} from its sums.  Inside the step graph
+// it runs in the body of the IF node on `second`, sets that back to 0 for the next Arnoldi step of
+// this index and counts the body's executions in *passes.
 static __global__ void gs_decide_kernel(SlotPtr<double> devp, SlotPtr<float> devfp, int nv,
-                                        int stage, const int32_t* run,
-                                        cudaGraphConditionalHandle second, int set_second,
-                                        unsigned long long* passes) {
-  if (stage == 2 && blockIdx.y == 0 && threadIdx.x == 0) {
+                                        const int32_t* run, cudaGraphConditionalHandle second,
+                                        int set_second, unsigned long long* passes) {
+  if (blockIdx.y == 0 && threadIdx.x == 0) {
     if (set_second) cudaGraphSetConditional(second, 0u);
     if (passes) ++*passes;
   }
@@ -981,35 +1148,19 @@ static __global__ void gs_decide_kernel(SlotPtr<double> devp, SlotPtr<float> dev
   double* __restrict__ dev = devp.at();
   float* __restrict__ devf = devfp.at();
   if (threadIdx.x != 0) {
-    // FP32 copies of the coefficients this stage produced (threads 1..)
-    const int base = stage == 1 ? 0 : kGsH2;
-    for (int k = threadIdx.x - 1; k < nv; k += blockDim.x - 1) devf[base + k] = (float)dev[base + k];
+    // FP32 copies of the coefficients (threads 1..)
+    for (int k = threadIdx.x - 1; k < nv; k += blockDim.x - 1) devf[kGsH2 + k] = (float)dev[kGsH2 + k];
     return;
   }
-  if (stage == 1) {
-    const double nw2 = dev[nv];
-    double s = 0.0;
-    for (int k = 0; k < nv; ++k) s = fma(dev[k], dev[k], s);
-    const double est = nw2 - s;
-    const bool reorth = !(est > kReorthTheta2 * nw2);
-    dev[kGsFlag] = reorth ? 1.0 : 0.0;
-    if (reorth && set_second) cudaGraphSetConditional(second, 1u);
-    const double hn = reorth ? 0.0 : sqrt(est);
-    dev[kGsNorm] = hn;
-    dev[kGsInv] = hn > 0.0 ? 1.0 / hn : 0.0;
-    devf[kGsFlag] = reorth ? 1.0f : 0.0f;
-    devf[kGsInv] = (float)dev[kGsInv];
-  } else {
-    if (dev[kGsFlag] == 0.0) return;
-    const double nw2 = dev[kGsH2 + nv];
-    double s = 0.0;
-    for (int k = 0; k < nv; ++k) s = fma(dev[kGsH2 + k], dev[kGsH2 + k], s);
-    const double e2 = nw2 - s;
-    const double hn = e2 > 0.0 ? sqrt(e2) : 0.0;
-    dev[kGsNorm] = hn;
-    dev[kGsInv] = hn > 0.0 ? 1.0 / hn : 0.0;
-    devf[kGsInv] = (float)dev[kGsInv];
-  }
+  if (dev[kGsFlag] == 0.0) return;
+  const double nw2 = dev[kGsH2 + nv];
+  double s = 0.0;
+  for (int k = 0; k < nv; ++k) s = fma(dev[kGsH2 + k], dev[kGsH2 + k], s);
+  const double e2 = nw2 - s;
+  const double hn = e2 > 0.0 ? sqrt(e2) : 0.0;
+  dev[kGsNorm] = hn;
+  dev[kGsInv] = hn > 0.0 ? 1.0 / hn : 0.0;
+  devf[kGsInv] = (float)dev[kGsInv];
 }
 
 enum GsMode { GS_FINAL1 = 0, GS_REORTH = 1, GS_FINAL2 = 2 };
@@ -1018,13 +1169,25 @@ enum GsMode { GS_FINAL1 = 0, GS_REORTH = 1, GS_FINAL2 = 2 };
 // a second pass) or h2 (FINAL2, runs with one); with an FP16 basis the new vector also goes to
 // outx in T (the preconditioner's input).  REORTH: w -= sum_k h_k V_k in place, with partial
 // V_k . w (rows k < NV) and |w|^2 (row NV) of the result.
+// (the registers of the Givens block must not cost the other blocks their residency: with an FP16
+// basis they need 34 to 44)
+template <class B, int MODE>
+constexpr int kGsBlocks = sizeof(B) == 2 && MODE != GS_REORTH ? 6 : 1;
 template <class T, class B, int NV, int MODE>
-__global__ void __launch_bounds__(256) gs_update_kernel(SlotPtr<B> outp, SlotPtr<T> outxp,
+__global__ void __launch_bounds__(256, kGsBlocks<B, MODE>) gs_update_kernel(SlotPtr<B> outp, SlotPtr<T> outxp,
                                                         SlotPtr<T> wp, SlotPtr<const B> Vp,
                                                         int64_t ldv, SlotPtr<const double> devp,
                                                         SlotPtr<const float> devfp, int64_t N,
-                                                        SlotPtr<double> pp, const int32_t* run) {
-  if (slot_idle(run)) return;
+                                                        SlotPtr<double> pp, const int32_t* run,
+                                                        const __grid_constant__ GivensArgs ga) {
+  // FINAL1: block 0 does the step's Givens updates (of every slot) beside the others
+  const int nblk = MODE == GS_FINAL1 ? (int)gridDim.x - 1 : (int)gridDim.x;
+  const int blk = MODE == GS_FINAL1 ? (int)blockIdx.x - 1 : (int)blockIdx.x;
+  if (MODE == GS_FINAL1 && blk < 0) {
+    if (blockIdx.y == 0) givens_block(ga, 0);
+    return;
+  }
+  if (MODE != GS_FINAL1 && slot_idle(run)) return;
   typedef typename AccType<T>::type A;
   typedef Pack16<T> P;
   typedef BasisIO<T, B> IO;
@@ -1033,7 +1196,7 @@ __global__ void __launch_bounds__(256) gs_update_kernel(SlotPtr<B> outp, SlotPtr
   constexpr bool kCopy = !std::is_same<T, B>::value;
   const A* cf = gs_coef<A>(devp.at(), devfp.at());
   const bool second = cf[kGsFlag] != A(0);
-  const bool runs = MODE == GS_FINAL1 ? !second : second;
+  const bool runs = MODE == GS_FINAL1 ? !second && cf[kGsOn] != A(0) : second;
   if (!runs) return;
   const A* coef = MODE == GS_FINAL2 ? cf + kGsH2 : cf;
   const A inv = cf[kGsInv];
@@ -1051,8 +1214,7 @@ __global__ void __launch_bounds__(256) gs_update_kernel(SlotPtr<B> outp, SlotPtr
 #pragma unroll
   for (int k = 0; k < NA; ++k) acc[k] = A(0);
   const int64_t ng = N / W;
-  for (int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; g < ng;
-       g += (int64_t)gridDim.x * blockDim.x) {
+  for (int64_t g = (int64_t)blk * blockDim.x + threadIdx.x; g < ng; g += (int64_t)nblk * blockDim.x) {
     A x[W];
 #pragma unroll
     for (int p = 0; p < NP; ++p) {
@@ -1108,7 +1270,7 @@ __global__ void __launch_bounds__(256) gs_update_kernel(SlotPtr<B> outp, SlotPtr
       }
     }
   }
-  if (blockIdx.x == 0 && threadIdx.x < N - ng * W) {  // the ragged tail
+  if (blk == 0 && threadIdx.x < N - ng * W) {  // the ragged tail
     const int64_t i = ng * W + threadIdx.x;
     A x = (A)w[i];
 #pragma unroll
@@ -1149,12 +1311,13 @@ template <class T, class B, int MODE>
 void launch_gs_update(int nvec, dim3 grid, cudaStream_t s, SlotPtr<B> out, SlotPtr<T> outx,
                       SlotPtr<T> w, SlotPtr<const B> V, int64_t ldv, SlotPtr<const double> dev,
                       SlotPtr<const float> devf, int64_t N, SlotPtr<double> partials,
-                      const int32_t* run) {
+                      const int32_t* run, const GivensArgs& ga) {
+  if (MODE == GS_FINAL1) ++grid.x;  // the block of the Givens updates
   switch (nvec) {
 #define BES_UPD_CASE(n)                                                                      \
   case n:                                                                                    \
     gs_update_kernel<T, B, n, MODE><<<grid, 256, 0, s>>>(out, outx, w, V, ldv, dev, devf, N, \
-                                                         partials, run);                     \
+                                                         partials, run, ga);                 \
     break;
     BES_NV_CASES(BES_UPD_CASE)
 #undef BES_UPD_CASE
@@ -1286,27 +1449,6 @@ struct SlotHandles {
   cudaGraphConditionalHandle h[kMaxSlots];  // IF of each slot's assembly and factorisation
 };
 
-struct GmresParam {
-  int mr;         // restart length
-  int maxiter;    // linear iteration limit
-  double tol;     // relative tolerance
-};
-
-struct GmresHandles {
-  cudaGraphConditionalHandle loop;              // WHILE over restart cycles
-  cudaGraphConditionalHandle arn[kMaxRestart];  // IF of Arnoldi step j
-  cudaGraphConditionalHandle gs2[kMaxRestart];  // IF of step j's second Gram-Schmidt pass
-  int on;                                       // 0: not inside a conditional graph
-};
-
-constexpr int kHsize = (kMaxRestart + 1) * kHld;  // Hessenberg entries per slot
-
-__device__ __forceinline__ void set_arnoldi_handles(const GmresHandles& h, int from, int mr,
-                                                    unsigned first) {
-  if (!h.on) return;
-  for (int k = from; k < mr; ++k) cudaGraphSetConditional(h.arn[k], k == from ? first : 0u);
-}
-
 // Start of slot t's solve: |b|^2 = nb2 gives beta; g = (beta, 0, ...), 1/beta for V_0 = b / beta.
 // Returns 1 if the solve runs.
 __device__ __forceinline__ int gmres_init_slot(const GmresDev& g, const GmresParam& P, int t,
@@ -1349,48 +1491,6 @@ static __global__ void gmres_init_kernel(GmresDev g, GmresParam P, GmresHandles 
     cudaGraphSetConditional(h.loop, any ? 1u : 0u);
     set_arnoldi_handles(h, 0, P.mr, any ? 1u : 0u);
   }
-}
-
-// Arnoldi step j, after the Gram-Schmidt kernels: column j of the Hessenberg matrix from the
-// slot's coefficients, the earlier Givens rotations applied to it, a new rotation that zeroes
-// h_{j+1,j}, and the rotated right-hand side; the slot's cycle stops when |g_{j+1}| <= eps,
-// at the restart length, or at the iteration limit.  Rotation arithmetic without FMA
-// contraction.
-static __global__ void gmres_givens_kernel(GmresDev g, GmresParam P, GmresHandles h, int nslot,
-                                           int j) {
-  const int t = threadIdx.x;
-  int cont = 0;
-  if (t < nslot && g.cyc[t]) {
-    double* H = g.H + (int64_t)t * kHsize;
-    double* cs = g.cs + (int64_t)t * kMaxRestart;
-    double* sn = g.sn + (int64_t)t * kMaxRestart;
-    double* gg = g.g + (int64_t)t * (kMaxRestart + 1);
-    const double* dev = g.dev + (int64_t)t * kGsLd;
-    const bool second = dev[kGsFlag] != 0.0;
-    if (second) ++g.second[t];
-    for (int i = 0; i <= j; ++i) H[i * kHld + j] = second ? __dadd_rn(dev[i], dev[kGsH2 + i]) : dev[i];
-    H[(j + 1) * kHld + j] = dev[kGsNorm];
-    for (int i = 0; i < j; ++i) {
-      const double a = H[i * kHld + j], b = H[(i + 1) * kHld + j];
-      H[i * kHld + j] = __dadd_rn(__dmul_rn(cs[i], a), __dmul_rn(sn[i], b));
-      H[(i + 1) * kHld + j] = __dadd_rn(__dmul_rn(-sn[i], a), __dmul_rn(cs[i], b));
-    }
-    const double a = H[j * kHld + j], c = H[(j + 1) * kHld + j];
-    const double d = sqrt(__dadd_rn(__dmul_rn(a, a), __dmul_rn(c, c)));
-    cs[j] = d == 0.0 ? 1.0 : a / d;
-    sn[j] = d == 0.0 ? 0.0 : c / d;
-    H[j * kHld + j] = d;
-    H[(j + 1) * kHld + j] = 0.0;
-    gg[j + 1] = __dmul_rn(-sn[j], gg[j]);
-    gg[j] = __dmul_rn(cs[j], gg[j]);
-    g.jc[t] = j + 1;
-    const int it = ++g.iter[t];
-    cont = (!(fabs(gg[j + 1]) <= g.sc[8 * t + 1]) && j + 1 < P.mr && it < P.maxiter) ? 1 : 0;
-    g.cyc[t] = cont;
-  }
-  const int any = __syncthreads_or(cont);
-  if (t == 0) ++g.counters[0];
-  if (t == 0 && j + 1 < P.mr) set_arnoldi_handles(h, j + 1, P.mr, any ? 1u : 0u);
 }
 
 // End of a cycle: y = H^{-1} g by back substitution over the slot's jc columns.
