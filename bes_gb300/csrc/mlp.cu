@@ -784,7 +784,9 @@ struct bes_mlp {
   bf16 *Wb[kLayers] = {}, *WT[kLayers] = {};  // BF16 copies of the hidden weights, as they are and transposed
   int64_t t = 0;             // AdamW steps taken
   double cmean[3] = {0, 0, 0}, csd[3] = {1, 1, 1}, oscale[kOut] = {1, 1, 1, 1, 1};
-  double* ustage = nullptr;  // one field [nc][5] on its way to or from the caller
+  double* ustage[2] = {};    // fields [nc][5] on their way to or from the caller
+  cudaStream_t copy = nullptr;               // the predictions' way out
+  cudaEvent_t ready[2] = {}, taken[2] = {};  // a field is complete, is copied
   // batch buffers (capacity in rows; transposed arrays have rows of `cap` values)
   int cap = 0;
   bf16 *H0 = nullptr, *H0T = nullptr;  // features of the batch
@@ -1024,8 +1026,13 @@ int bes_mlp_create(const bes_ctx* ctx, uint64_t seed, bes_mlp** out) {
   bes_mlp* h = new bes_mlp();
   h->device = ctx->device;
   cudaSetDevice(h->device);
-  if (cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking) != cudaSuccess) {
-    delete h;
+  bool made = cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking) == cudaSuccess &&
+              cudaStreamCreateWithFlags(&h->copy, cudaStreamNonBlocking) == cudaSuccess;
+  for (int b = 0; b < 2 && made; ++b)
+    made = cudaEventCreateWithFlags(&h->ready[b], cudaEventDisableTiming) == cudaSuccess &&
+           cudaEventCreateWithFlags(&h->taken[b], cudaEventDisableTiming) == cudaSuccess;
+  if (!made) {
+    bes_mlp_destroy(h);
     return BES_ERR_CUDA;
   }
   h->gamma = ctx->opt.specific_heat_ratio;
@@ -1057,7 +1064,7 @@ int bes_mlp_create(const bes_ctx* ctx, uint64_t seed, bes_mlp** out) {
     rc |= mlp_alloc(h, &h->Wb[l], (size_t)kW * (l == 0 ? kK0 : kW));
     rc |= mlp_alloc(h, &h->WT[l], (size_t)kW * (l == 0 ? kK0 : kW));
   }
-  rc |= mlp_alloc(h, &h->ustage, (size_t)h->nc * kOut);
+  for (double*& u : h->ustage) rc |= mlp_alloc(h, &u, (size_t)h->nc * kOut);
   rc |= mlp_alloc(h, &h->gemm_err, 1);
   rc |= set_smem_limits(h);
   if (rc) {
@@ -1098,9 +1105,15 @@ int bes_mlp_create(const bes_ctx* ctx, uint64_t seed, bes_mlp** out) {
 
 void bes_mlp_destroy(bes_mlp* h) {
   if (!h) return;
-  if (h->stream) cudaStreamSynchronize(h->stream);
+  for (cudaStream_t s : {h->stream, h->copy})
+    if (s) cudaStreamSynchronize(s);
   for (void* q : h->allocs) cudaFree(q);
-  if (h->stream) cudaStreamDestroy(h->stream);
+  for (int b = 0; b < 2; ++b) {
+    if (h->ready[b]) cudaEventDestroy(h->ready[b]);
+    if (h->taken[b]) cudaEventDestroy(h->taken[b]);
+  }
+  for (cudaStream_t s : {h->stream, h->copy})
+    if (s) cudaStreamDestroy(s);
   delete h;
 }
 
@@ -1237,8 +1250,8 @@ int bes_mlp_train(bes_mlp* h, int32_t n_samples, const double* mach, const doubl
   cudaMemcpyAsync(dscale, scale.data(), scale.size() * 8, cudaMemcpyHostToDevice, h->stream);
   for (int q = 0; q < n_samples; ++q) {
     const int64_t n = nc * kOut;
-    cudaMemcpyAsync(h->ustage, U + (size_t)q * n, n * sizeof(double), cudaMemcpyHostToDevice, h->stream);
-    targets_kernel<<<1024, 256, 0, h->stream>>>(n, n, h->ustage, dscale + q * kOut,
+    cudaMemcpyAsync(h->ustage[0], U + (size_t)q * n, n * sizeof(double), cudaMemcpyHostToDevice, h->stream);
+    targets_kernel<<<1024, 256, 0, h->stream>>>(n, n, h->ustage[0], dscale + q * kOut,
                                                 dscale + n_samples * kOut, dt + (size_t)q * n);
   }
   const size_t n_lp = (batch + 255) / 256;
@@ -1277,16 +1290,29 @@ int bes_mlp_infer(bes_mlp* h, int32_t n, const double* mach, double* U) {
   if (!h || !mach || !U || n < 0) return BES_ERR_INVALID;
   ForwardArgs a = forward_args(h);
   a.X = h->feat;
-  a.U = h->ustage;
   a.n = h->nc;
   for (int v = 0; v < kOut; ++v) a.oscale[v] = h->oscale[v];
-  for (int q = 0; q < n; ++q) {
-    for (int d = 0; d < 3; ++d) a.c3[d] = (float)((mach[q * 3 + d] - h->cmean[d]) / h->csd[d]);
-    freestream_conserved(h->gamma, h->R, &mach[q * 3], a.Uinf);
-    launch_forward<false>(h, a, h->n_rows);
-    MLP_TRY(h, cudaMemcpyAsync(U + (size_t)q * h->nc * kOut, h->ustage, (size_t)h->nc * kOut * sizeof(double),
-                               cudaMemcpyDeviceToHost, h->stream));
+  // The copy to the caller's memory takes longer than the kernel (pageable memory, and the call
+  // returns when it is done): the next condition's kernel is launched before it, on the other field.
+  for (int q = 0; q <= n; ++q) {
+    if (q < n) {
+      const int b = q & 1;
+      for (int d = 0; d < 3; ++d) a.c3[d] = (float)((mach[q * 3 + d] - h->cmean[d]) / h->csd[d]);
+      freestream_conserved(h->gamma, h->R, &mach[q * 3], a.Uinf);
+      a.U = h->ustage[b];
+      if (q >= 2) MLP_TRY(h, cudaStreamWaitEvent(h->stream, h->taken[b], 0));
+      launch_forward<false>(h, a, h->n_rows);
+      MLP_TRY(h, cudaEventRecord(h->ready[b], h->stream));
+    }
+    if (q > 0) {
+      const int b = (q - 1) & 1;
+      MLP_TRY(h, cudaStreamWaitEvent(h->copy, h->ready[b], 0));
+      MLP_TRY(h, cudaMemcpyAsync(U + (size_t)(q - 1) * h->nc * kOut, h->ustage[b],
+                                 (size_t)h->nc * kOut * sizeof(double), cudaMemcpyDeviceToHost, h->copy));
+      MLP_TRY(h, cudaEventRecord(h->taken[b], h->copy));
+    }
   }
+  MLP_TRY(h, cudaStreamSynchronize(h->copy));
   MLP_TRY(h, cudaStreamSynchronize(h->stream));
   MLP_TRY(h, cudaGetLastError());
   return gemm_status(h);
