@@ -177,15 +177,14 @@ WORKLOADS = {
 }
 
 # bytes each kernel must move per unit (compulsory traffic of the SoA layout, FP64):
-#   cell sweep per cell: state of the cell (40) + Sc (96) + w (32) + r (96) + adj (16)
-#     + flags (1) + 1/V (8) + eps^2 (8) + face-side state written (40)      = 337
-#     (stage 0 adds plen 24 + V 8 + dt 8 = 40; neighbour states are re-reads of the same array)
-#   face flux per face: RS indices (8) + normal (24) + area (8) + two side states (80)
-#     + flux x area written (40)                                            = 160
+#   cell sweep per cell: state (40) + 4x4 gradient matrix (128) + adj (16) + flags (1)
+#     + eps^2 (8) + one side state of eight values written (64)              = 257
+#   face flux per face: state indices (8) + normal (24) + area (8) + two side states (128)
+#     + flux x area written (40)                                            = 208
 #   update per cell: 4 face ids (16) + 4 fluxes (160) + U(n) (40) + dt (8) + 1/V (8)
 #     + U written (40)                                                      = 272
-BYTES_PER_CELL_SWEEP = 337.0
-BYTES_PER_FACE = 160.0
+BYTES_PER_CELL_SWEEP = 257.0
+BYTES_PER_FACE = 208.0
 BYTES_PER_UPDATE = 272.0
 
 
@@ -388,10 +387,10 @@ def run_reference(args, wl):
 #     and written in both sweeps (4 x 20)                                          = 580
 #   matrix-vector product: five blocks (500) + x (20) + y (20)                       = 540
 # With an FP64 system the block and vector bytes double.  With 16-bit block-scaled storage
-# (precision 2) a block is 13 half2 words + one FP32 scale = 56 bytes: preconditioner
-# 5 x 56 + 80 = 360, matrix-vector product 5 x 56 + 40 = 320.
-BYTES_PRECOND = {2: 360.0, 1: 580.0, 0: 1160.0}
-BYTES_SPMV = {2: 320.0, 1: 540.0, 0: 1080.0}
+# (precision 2) a block is 13 words = 52 bytes: preconditioner 5 x 52 + 80 = 340, matrix-vector
+# product 5 x 52 + 40 = 300.
+BYTES_PRECOND = {2: 340.0, 1: 580.0, 0: 1160.0}
+BYTES_SPMV = {2: 300.0, 1: 540.0, 0: 1080.0}
 KERNEL_NAMES = {
     "precond": {2: "block-ILU(0) colour sweeps, packed blocks (ilu_colour_packed_kernel)",
                 1: "block-ILU(0) colour sweeps (ilu_colour_kernel)",
@@ -407,6 +406,10 @@ FLOPS_PER_CELL_STAGE = 646  # cell sweep 614 (gradient 184, 1/V 15, limiter 370,
 FLOPS_PER_CELL_DT = 33      # local time step, once per iteration
 FLOPS_PER_UPDATE = 32       # update kernel per cell and stage (part of FLOPS_PER_CELL_STAGE)
 FLOPS_PER_FACE_STAGE = 186  # Roe flux 181 + flux x area 5 (boundary faces need fewer)
+# FP64 instructions that the explicit kernels issue per unit and stage (their algebra needs fewer
+# operations than the formulas counted above; csrc/side_kernels.cuh): the FP64 pipe takes the same
+# time for each, so the kernels' roofline is this count against the measured instruction rate
+FP64_INSTR = {"side_recon_kernel": 180.0, "side_flux_kernel": 77.5, "update_kernel": 27.0}
 
 
 def explicit_fp64_work(nc: int, nf: int, cell_updates_per_s: float, n_stage: int = 4) -> dict:
@@ -1207,21 +1210,19 @@ def main():
     e2e = world * ncond * nc * args.steps / e2e_max
 
     n_stage = 4
-    per_launch = {"cell_recon_kernel": kms[0] / (args.steps * n_stage),
-                  "face_flux_kernel": kms[1] / (args.steps * n_stage),
+    per_launch = {"side_recon_kernel": kms[0] / (args.steps * n_stage),
+                  "side_flux_kernel": kms[1] / (args.steps * n_stage),
                   "update_kernel": kms[2] / (args.steps * n_stage)}
-    bytes_per_launch = {"cell_recon_kernel": BYTES_PER_CELL_SWEEP * nc * ncond,
-                        "face_flux_kernel": BYTES_PER_FACE * nf * ncond,
+    bytes_per_launch = {"side_recon_kernel": BYTES_PER_CELL_SWEEP * nc * ncond,
+                        "side_flux_kernel": BYTES_PER_FACE * nf * ncond,
                         "update_kernel": BYTES_PER_UPDATE * nc * ncond}
     dom = max(per_launch, key=lambda k: per_launch[k])
     peak, peak_kind = measured_peaks()
     achieved = bytes_per_launch[dom] / (per_launch[dom] / 1e3) / 1e9
-    # the explicit kernels move about one FP64 flop per byte, far above this GPU's FP64 ridge
-    # point: their bound is the FP64 pipe (counted flops over the measured FMA rate x 2)
-    flops_per_launch = {"cell_recon_kernel": (FLOPS_PER_CELL_STAGE - FLOPS_PER_UPDATE
-                                              + FLOPS_PER_CELL_DT / n_stage) * nc * ncond,
-                        "face_flux_kernel": FLOPS_PER_FACE_STAGE * nf * ncond,
-                        "update_kernel": FLOPS_PER_UPDATE * nc * ncond}
+    # the explicit kernels are bound by the FP64 pipe: instructions issued (two flops each, as
+    # an FMA) against the measured FMA rate x 2
+    flops_per_launch = {k: 2.0 * n * (nf if k == "side_flux_kernel" else nc) * ncond
+                        for k, n in FP64_INSTR.items()}
     fp64_peak = 2.0 * lib.fp64_fma_rate() / 1e12
     fp64_achieved = flops_per_launch[dom] / (per_launch[dom] / 1e3) / 1e12
     roof = {"kernel": dom, "bound": "fp64", "achieved": fp64_achieved, "peak": fp64_peak,
@@ -1232,8 +1233,8 @@ def main():
             "ms_per_launch": per_launch[dom], "flops_per_launch": flops_per_launch[dom],
             "hbm": {"achieved_gbs": achieved, "peak_gbs": peak, "frac": achieved / peak,
                     "bytes_per_launch": bytes_per_launch[dom], "peak_source": peak_kind},
-            "kernel_ms_per_step": {"cell_recon_kernel": kms[0] / args.steps,
-                                   "face_flux_kernel": kms[1] / args.steps,
+            "kernel_ms_per_step": {"side_recon_kernel": kms[0] / args.steps,
+                                   "side_flux_kernel": kms[1] / args.steps,
                                    "update_kernel": kms[2] / args.steps}}
     line = {"metric": METRIC, "metric_full": METRIC_FULL, "value": value, "unit": METRIC,
             "n_gpus": world, "steps": args.steps, "warmup": args.warmup,

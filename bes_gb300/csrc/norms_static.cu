@@ -4,8 +4,8 @@
 // already reserved the device memory it will use (a raw cudaMalloc there can fail or
 // fragment the pool), or a latency-critical loop in which a cudaMalloc/cudaFree pair would
 // synchronise the whole device.  For them bes_residual_norms_static computes the per-variable
-// L2 and max norms of a residual with the same two-kernel reduction the explicit iteration
-// uses at its last stage, but keeps the per-block partial sums in a fixed array of device
+// L2 and max norms of a residual with a two-kernel reduction as the explicit iteration has at its
+// last stage, but keeps the per-block partial sums in a fixed array of device
 // memory owned by this file instead of in a buffer from cudaMalloc.  The caller passes the
 // residual and the output, both already in device memory.
 #include <cuda_runtime.h>
@@ -66,8 +66,7 @@ __device__ __forceinline__ double wmax(double x) {
   return x;
 }
 
-// Same block reduction as the last-stage update of the explicit iteration, reading a
-// residual stored cell-major [n][5].
+// Block partials of the norms of a residual stored cell-major [n][5].
 __global__ void __launch_bounds__(kNormBlock) static_norm_partial_kernel(
     const double* __restrict__ R, int64_t n, double* __restrict__ partials) {
   const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
