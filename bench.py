@@ -419,8 +419,8 @@ def explicit_fp64_work(nc: int, nf: int, cell_updates_per_s: float, n_stage: int
     per_cell = per_iter / nc
     return {"flops_per_cell_update": per_cell,
             "achieved_tflops": cell_updates_per_s * per_cell / 1e12,
-            "note": "add/sub/mul counted once each (divisions and square roots on top); the "
-                    "cell sweep and the face flux are FP64-issue bound on this GPU"}
+            "note": "of the formulas: add/sub/mul counted once each (divisions and square roots "
+                    "on top); the kernels issue fewer (roofline) and are FP64-issue bound"}
 
 
 def implicit_leg(args, torch, ctx, steps, warmup, flush, with_e2e, prof_steps: int = 5):
