@@ -60,6 +60,10 @@ __device__ __forceinline__ double fast_rsqrt(double x) {
   const double e = fma(-x * y, y, 1.0);
   return fma(y * e, fma(e, 0.375, 0.5), y);
 }
+// sqrt(x) by the same; sqrt(0) is 0 (0 * 1/sqrt(0) is a NaN: a cell without pressure is a valid state)
+__device__ __forceinline__ double fast_sqrt(double x) {
+  return mid_range(x) ? x * fast_rsqrt(x) : sqrt(x);
+}
 __device__ __forceinline__ long long dbits(double x) { return __double_as_longlong(x); }
 // a <= b for a, b >= 0 (or a NaN, which compares greater than every number)
 __device__ __forceinline__ bool le_nonneg(double a, double b) { return dbits(a) <= dbits(b); }
@@ -130,7 +134,7 @@ __device__ __forceinline__ double local_time_step(const DevMesh& m, const Params
   for (int d = 0; d < 3; ++d) w[d] = u[1 + d] * ir;
   const double k = fma(u[1], w[0], fma(u[2], w[1], u[3] * w[2]));
   const double cs2 = g.gamma2_gm1 * fma(-0.5, k, u[4]) * ir;
-  const double cs = cs2 * fast_rsqrt(cs2);
+  const double cs = fast_sqrt(cs2);
   double spec = 0.0;
 #pragma unroll
   for (int d = 0; d < 3; ++d) spec = fma(cs + fabs(w[d]), m.plen[(int64_t)d * m.nc + c], spec);
