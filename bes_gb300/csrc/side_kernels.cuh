@@ -103,9 +103,17 @@ static __global__ void __launch_bounds__(128) face_matrix_kernel(DevMesh m, doub
 __device__ __forceinline__ void store_side(const Params& g, const double* x, double* __restrict__ dst) {
   SideState q;
   q.rho = 0.5 * x[0];
-  const double y = fast_rsqrt(q.rho);
-  q.s = q.rho * y;
-  const double ir = 0.5 * (y * y);
+  double ir;
+  if (mid_range(q.rho)) {
+    const double y = fast_rsqrt(q.rho);
+    q.s = q.rho * y;
+    ir = 0.5 * (y * y);
+  } else {
+    // a density extrapolated below 0 at a wall face has a pressure all the same, which is all
+    // that the wall's flux takes; only the Roe flux takes its root (a NaN)
+    q.s = sqrt(q.rho);
+    ir = 1.0 / x[0];
+  }
 #pragma unroll
   for (int d = 0; d < 3; ++d) q.u[d] = x[1 + d] * ir;
   const double k = fma(x[1], q.u[0], fma(x[2], q.u[1], x[3] * q.u[2]));

@@ -45,3 +45,20 @@ def test_cell_without_pressure(mesh, local, exact):
     U0 = _uniform(mesh, mach)
     U0[mesh.n_cells // 2, 4] = 0.5 * 0.5 ** 2
     _compare(mesh, U0, mach, local, exact, 3, 0.5)
+
+
+@pytest.mark.parametrize("mesh,cell,low", [(meshgen.bump_channel(5, 1, 1, 0.04), 1, 0.004),
+                                           (meshgen.bump_channel(9, 3, 1, 0.08), 100, 0.02),
+                                           (meshgen.bump_channel_2d(13, 5, 0.08), 10, 0.02)])
+def test_density_below_zero_at_a_wall_face(mesh, cell, low):
+    """A light cell at a wall: the density extrapolated to the wall's face (no face values limit it)
+    is negative, the pressure there is not, and the wall's flux takes the pressure only."""
+    mach = (0.5, 0.0, 0.0)
+    U0 = _uniform(mesh, mach)
+    U0[cell, 4] += 0.5 * (low - 1.0) * 0.5 ** 2
+    U0[cell, :4] *= low
+    O = pyoracle.Oracle(mesh, cfl=0.05, mach=mach, local_dt=1, muscl_exact=1)
+    O.set_state(U0)
+    below = O.operators(0.05)["face_UL"][:, 0] < 0
+    assert below.any() and (lib.host_geometry(mesh)["face_type"][below] == 1).all()
+    _compare(mesh, U0, mach, 1, 1, 1, 0.05)
