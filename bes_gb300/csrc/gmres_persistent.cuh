@@ -156,6 +156,14 @@ __device__ __forceinline__ double ld_relaxed(const double* p) {
   asm volatile("ld.relaxed.gpu.global.f64 %0, [%1];" : "=d"(v) : "l"(p) : "memory");
   return v;
 }
+// An entry that other blocks may be polling: a strong store, as their loads are (a weak one beside
+// them would be a data race).
+__device__ __forceinline__ void st_relaxed(float* p, float v) {
+  asm volatile("st.relaxed.gpu.global.f32 [%0], %1;" : : "l"(p), "f"(v) : "memory");
+}
+__device__ __forceinline__ void st_relaxed(double* p, double v) {
+  asm volatile("st.relaxed.gpu.global.f64 [%0], %1;" : : "l"(p), "d"(v) : "memory");
+}
 // gather5 of entries that may not be there yet; false while one is missing
 __device__ __forceinline__ bool try_gather5(const float* x, int j, float* y) {
   const int64_t e0 = (int64_t)j * 5;
@@ -219,7 +227,7 @@ __device__ __forceinline__ T wait_entry(const T* x, int* error) {
 }
 template <class T>
 __device__ __forceinline__ void put_entry(T* x, T v) {
-  __stcg(x, is_mark(v) ? Mark<T>::nan() : v);
+  st_relaxed(x, is_mark(v) ? Mark<T>::nan() : v);
 }
 
 // ---- rows ----------------------------------------------------------------------------------------
