@@ -789,7 +789,7 @@ int end_step(const Sys<T, B>& S, cudaStream_t s0, int prof, cudaGraph_t* out) {
   ImplicitBuffers& I = c->imp;
   stamp(c, s0, PROF_OTHER, 1);
   state_update_kernel<T><<<S.vgrid, 256, 0, s0>>>(slots(c->U[c->cur], 5LL * S.nc), S.cvec(S.X),
-                                                  (int64_t)S.nc, c->nan_flag, I.act);
+                                                  (int64_t)S.nc, c->nan_flag, I.sync_error, I.act);
   stamp(c, s0, PROF_OTHER, 0);
   IMP_TRY(c, cudaGetLastError());
   IMP_TRY(c, cudaStreamEndCapture(s0, out));
@@ -963,8 +963,8 @@ int run_steps(bes_ctx* c, int64_t n, double* history) {
     ++I.host_syncs;
     if (sync_err) {
       if ((rc = reset_grid_sync(c))) return rc;
-      c->last_error = "a grid barrier of the persistent colour sweep gave up after one second; "
-                      "the step's linear solves are not valid";
+      check_step_nan(c, nan);  // the flag is the failed step's
+      c->last_error = "a wait of the linear solves gave up after one second; the step was not applied";
       return BES_ERR_TIMEOUT;
     }
     // kernels this step launched: the graph's top level, the assembly of each slot that
@@ -1291,6 +1291,15 @@ int bes_set_linear_guard(bes_ctx* ctx, int32_t max_cycles) {
   ctx->imp.guard = max_cycles;
   IMP_TRY(ctx, cudaMemcpyAsync(ctx->imp.guard_dev, &ctx->imp.guard, sizeof(int32_t),
                                cudaMemcpyHostToDevice, ctx->stream));
+  IMP_TRY(ctx, cudaStreamSynchronize(ctx->stream));
+  return BES_OK;
+}
+
+int bes_inject_failure(bes_ctx* ctx, int32_t what) {
+  if (!ctx || what != BES_FAIL_WAIT) return BES_ERR_INVALID;
+  if (ctx->opt.solver_type != 1 || !ctx->imp.sync_error) return BES_ERR_INVALID;
+  const int on = 1;
+  IMP_TRY(ctx, cudaMemcpyAsync(ctx->imp.sync_error, &on, sizeof(int), cudaMemcpyHostToDevice, ctx->stream));
   IMP_TRY(ctx, cudaStreamSynchronize(ctx->stream));
   return BES_OK;
 }

@@ -1416,12 +1416,14 @@ __global__ void __launch_bounds__(256) zero_kernel(SlotPtr<T> xp, int64_t N, con
 }
 
 // state update W += dW (SolverImplicit::updateSolution_, src/SolverImplicit.cpp:509-528), for
-// every slot that took the step; skipped entirely when a face flux was NaN (the step fails)
+// every slot that took the step; skipped entirely when a face flux was NaN or a wait of the linear
+// solves gave up (the step fails)
 template <class T>
 __global__ void __launch_bounds__(256) state_update_kernel(SlotPtr<double> Up, SlotPtr<const T> dWp,
                                                            int64_t nc, const int* nan_flag,
+                                                           const int* sync_error,
                                                            const int32_t* run) {
-  if (slot_idle(run) || *nan_flag) return;
+  if (slot_idle(run) || *nan_flag || *sync_error) return;
   // U is [5][nc] (the solver's layout), dW cell-major [nc][5] (the Krylov layout)
   double* __restrict__ U = Up.at();
   const T* __restrict__ dW = dWp.at();

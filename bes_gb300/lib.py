@@ -30,7 +30,7 @@ EXPORTED = [
     "bes_output_default", "bes_output_from_besi", "bes_write", "bes_write_host", "bes_solve",
     "bes_create_batch", "bes_conditions", "bes_set_active", "bes_sweep_run",
     "bes_implicit_stats", "bes_set_linear_guard", "bes_set_condition", "bes_implicit_sweep",
-    "bes_tuning", "bes_fp64_fma_rate", "bes_host_layout_digest", "bes_checkpoint_save",
+    "bes_inject_failure", "bes_tuning", "bes_fp64_fma_rate", "bes_host_layout_digest", "bes_checkpoint_save",
     "bes_checkpoint_load",
     "bes_mlp_create", "bes_mlp_destroy", "bes_mlp_last_error", "bes_mlp_train", "bes_mlp_infer",
     "bes_mlp_init_state", "bes_mlp_params", "bes_mlp_features", "bes_mlp_loss_grad",
@@ -38,6 +38,7 @@ EXPORTED = [
 ]
 
 OUTPUT_VTK, OUTPUT_CSV, OUTPUT_SLIP_WALL_CSV = 0, 1, 2
+FAIL_WAIT = 1
 
 
 class BesError(RuntimeError):
@@ -143,6 +144,7 @@ def load(path: str = LIB_PATH):
                                 ctypes.POINTER(ctypes.c_int64), D]
     L.bes_implicit_stats.argtypes = [P, ctypes.POINTER(ctypes.c_int64)]
     L.bes_set_linear_guard.argtypes = [P, ctypes.c_int32]
+    L.bes_inject_failure.argtypes = [P, ctypes.c_int32]
     L.bes_tuning.argtypes = [P, ctypes.c_char_p, ctypes.c_size_t]
     L.bes_fp64_fma_rate.argtypes = [D]
     L.bes_checkpoint_save.argtypes = [P, ctypes.c_char_p]
@@ -522,6 +524,10 @@ class Context:
     def set_linear_guard(self, max_cycles: int):
         """bes_set_linear_guard: restart-cycle limit of one linear solve (0: default)."""
         self._check(load().bes_set_linear_guard(self.h, int(max_cycles)))
+
+    def inject_failure(self, what: int):
+        """bes_inject_failure: a failure made on the host for the next implicit step (FAIL_*)."""
+        self._check(load().bes_inject_failure(self.h, int(what)))
 
     def set_condition(self, cond: int, mach=None, U=None):
         """bes_set_condition: a new condition (Mach vector, state or freestream) in slot cond."""

@@ -161,8 +161,9 @@ int bes_explicit_iterations(bes_ctx* ctx, int64_t n, double* history);
  * linear iterations, final relative linear residual, L2[5] of the unscaled residual
  * R = sum(+-F A) (the convergence measure).  A frozen condition (bes_set_active) does not
  * step; its history rows are zeros.  Returns BES_ERR_TIMEOUT when a linear solve was stopped
- * by its restart-cycle limit (bes_set_linear_guard); the step is applied and the context stays
- * usable. */
+ * by its restart-cycle limit (bes_set_linear_guard), with the step applied, or when a wait
+ * between the blocks of a persistent kernel gave up, with the state as it was before the step; the
+ * context stays usable. */
 int bes_implicit_steps(bes_ctx* ctx, int64_t n, double* history);
 
 /* Implicit-path statistics: out[0] steps taken, out[1] host synchronisations inside
@@ -179,6 +180,12 @@ int bes_tuning(const bes_ctx* ctx, char* buf, size_t cap);
  * returns BES_ERR_TIMEOUT.  The device loop over restart cycles ends by construction; this
  * bound is its guard and lets a caller cap the work of one step. */
 int bes_set_linear_guard(bes_ctx* ctx, int32_t max_cycles);
+
+/* Test aid: a failure made on the host, for the context's next implicit step.
+ *   BES_FAIL_WAIT  the flag that a wait of the linear solves sets when it gives up is set before
+ *                  the step: the step is not applied and returns BES_ERR_TIMEOUT. */
+#define BES_FAIL_WAIT 1
+int bes_inject_failure(bes_ctx* ctx, int32_t what);
 
 /* Assemble (without solving or updating) the implicit system at the current state and CFL
  * (SolverImplicit::computeFaceFluxes_ and the CoefficientMatrix, src/SolverImplicit.cpp:358-507).

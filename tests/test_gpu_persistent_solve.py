@@ -1,8 +1,9 @@
-"""The one-launch linear solve (GPU): rows wait for entries that other blocks write."""
+"""The one-launch linear solve (GPU): rows wait for entries that other blocks write, and a failure (made
+on the host) leaves the context usable."""
 import numpy as np
 import pytest
 
-from bes_gb300 import meshgen
+from bes_gb300 import lib, meshgen
 from tests._gpu import context
 
 pytestmark = pytest.mark.gpu
@@ -25,3 +26,32 @@ def test_repeated_solves_are_equal(precision, linear):
     ctx.close()
     for h, U in runs[1:]:
         assert np.array_equal(h, runs[0][0]) and np.array_equal(U, runs[0][1])
+
+
+@pytest.mark.parametrize("precision", [0, 1, 2])
+@pytest.mark.parametrize("sweep_kernel", [0, 2])
+@pytest.mark.parametrize("n_cond", [1, 3])
+def test_step_whose_wait_gave_up_is_not_applied(precision, sweep_kernel, n_cond):
+    """The second step fails: the state stays the first step's, and the next step is the second."""
+    mesh = meshgen.bump_channel(9, 3, 1, 0.08)
+    machs = np.array([[0.5, 0.02, 0.0], [0.7, 0.0, 0.0], [0.6, 0.0, 0.03]])[:n_cond]
+
+    def ctx():
+        o = lib.default_options(precision=precision, linear_solver=1, sweep_kernel=sweep_kernel, **OPTS)
+        return lib.Context(mesh, o, machs=machs if n_cond > 1 else None)
+
+    plain = ctx()
+    plain.implicit_steps(1)
+    U1 = plain.get_state()
+    h2, U2 = plain.implicit_steps(1), plain.get_state()
+    plain.close()
+    c = ctx()
+    c.implicit_steps(1)
+    c.inject_failure(lib.FAIL_WAIT)
+    with pytest.raises(lib.BesError) as e:
+        c.implicit_steps(1)
+    assert e.value.code == 7
+    assert np.array_equal(c.get_state(), U1)
+    assert np.array_equal(c.implicit_steps(1), h2)
+    assert np.array_equal(c.get_state(), U2)
+    c.close()
