@@ -166,9 +166,11 @@ struct ImplicitBuffers {
   // resident blocks with a bounded grid barrier between colours); chosen by the autotuner on
   // the first step unless the options fix it
   int sweep_kernel = 1;        // 1 per colour, 2 persistent, 3 per colour with loads first
+  int inject = 0;              // BES_FAIL_* of the next step graph
   bool tuned = false;
   int persistent_blocks = 0;   // grid of the persistent sweep
   int solve_blocks = 0;        // grid of the persistent linear solve; 0: the step graph's solve
+  bool solve_dropped = false;  // it was refused or a wait of it gave up: not taken again
   bool solve_lane_spmv = false;  // the row form of its products
   void* Y = nullptr;           // its forward-solve vector [ldv], per condition
   int solve_resident = 0;      // blocks of it that can be resident

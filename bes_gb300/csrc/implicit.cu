@@ -254,7 +254,12 @@ cudaError_t launch_persistent_sweep(const Sys<T, B>& S, cudaStream_t s, SlotPtr<
 template <class T, class B>
 int enqueue_persistent_solve(const Sys<T, B>& S, cudaStream_t s, const GmresParam& P, int prof) {
   bes_ctx* c = S.c;
-  const ImplicitBuffers& I = c->imp;
+  ImplicitBuffers& I = c->imp;
+  if (I.inject == BES_FAIL_SOLVE_CAPTURE) {
+    I.inject = 0;
+    c->last_error = "the one-launch linear solve was refused";
+    return BES_ERR_CUDA;
+  }
   SolveArgs<T, B> a;
   std::memset(&a, 0, sizeof(a));
   a.m = c->dm;
@@ -626,7 +631,8 @@ void choose_solve(bes_ctx* c) {
   ImplicitBuffers& I = c->imp;
   I.solve_blocks = 0;
   SweepPlan plan;
-  if (c->opt.sweep_kernel != 0 || c->opt.linear_solver == 2 || I.solve_resident < 1) return;
+  if (c->opt.sweep_kernel != 0 || c->opt.linear_solver == 2 || I.solve_resident < 1 || I.solve_dropped)
+    return;
   if (uses_ilu(c) && (!I.use_colour_ranges || !sweep_plan(c->soa, plan))) return;
   const int64_t rows = (int64_t)c->soa.nc * I.nslot;
   int64_t stage = rows;
@@ -848,29 +854,13 @@ int capture_step(bes_ctx* c, int prof, cudaGraph_t* out) {
   return end_step(S, s0, prof, out);
 }
 
+// The step's executable graph in the forms that are chosen; after a failure the streams are usable.
 template <class T, class B>
-int build_step_graph(bes_ctx* c, int prof) {
+int make_step_graph(bes_ctx* c, int prof) {
   ImplicitBuffers& I = c->imp;
-  if (!I.cap[0]) {
-    IMP_TRY(c, cudaStreamCreateWithFlags(&I.cap[0], cudaStreamNonBlocking));
-    IMP_TRY(c, cudaStreamCreateWithFlags(&I.cap[1], cudaStreamNonBlocking));
-    IMP_TRY(c, cudaStreamCreateWithFlags(&I.cap[2], cudaStreamNonBlocking));
-  }
-  if (!I.tuned) {
-    const int rc = tune_sweep<T, B>(c);
-    if (rc) return rc;
-  }
   cudaGraph_t g = nullptr;
   t_stamps = prof != 0;
-  int rc = capture_step<T, B>(c, prof, &g);
-  if (rc && I.sweep_kernel == 2) {
-    // the persistent launch could not be captured: one launch per colour
-    abandon_capture(c);
-    I.sweep_kernel = 1;
-    I.tuning += "colour sweep: the persistent launch could not be captured in the step graph; "
-                "taken: one launch per colour\n";
-    rc = capture_step<T, B>(c, prof, &g);
-  }
+  const int rc = capture_step<T, B>(c, prof, &g);
   t_stamps = false;
   if (rc) {
     abandon_capture(c);
@@ -879,11 +869,50 @@ int build_step_graph(bes_ctx* c, int prof) {
   const cudaError_t e = cudaGraphInstantiate(&I.step_graph[prof][c->cur], g, 0);
   cudaGraphDestroy(g);
   if (e != cudaSuccess) {
+    cudaGetLastError();
     c->last_error = std::string("cudaGraphInstantiate (implicit step): ") + cudaGetErrorString(e);
     I.step_graph[prof][c->cur] = nullptr;
     return BES_ERR_CUDA;
   }
   return BES_OK;
+}
+
+// The persistent kernels are an option, the step graph's solve with one launch per colour always
+// runs: after a refusal, or a wait that gave up, the context goes on with that.  The step graphs
+// made so far (none is running) are made again.
+void drop_persistent(bes_ctx* c, const char* why) {
+  ImplicitBuffers& I = c->imp;
+  for (auto& graphs : I.step_graph)
+    for (cudaGraphExec_t& g : graphs) {
+      if (g) cudaGraphExecDestroy(g);
+      g = nullptr;
+    }
+  if (I.solve_blocks > 0) {
+    I.solve_blocks = 0;
+    I.solve_dropped = true;
+    I.tuned = false;  // the colour sweeps have not been timed
+    I.tuning += std::string("linear solves: the persistent launch ") + why + "; taken: the step graph's solve\n";
+  } else if (I.sweep_kernel == 2) {
+    I.sweep_kernel = 1;
+    I.tuning += std::string("colour sweep: the persistent launch ") + why + "; taken: one launch per colour\n";
+  }
+}
+
+template <class T, class B>
+int build_step_graph(bes_ctx* c, int prof) {
+  ImplicitBuffers& I = c->imp;
+  if (!I.cap[0]) {
+    IMP_TRY(c, cudaStreamCreateWithFlags(&I.cap[0], cudaStreamNonBlocking));
+    IMP_TRY(c, cudaStreamCreateWithFlags(&I.cap[1], cudaStreamNonBlocking));
+    IMP_TRY(c, cudaStreamCreateWithFlags(&I.cap[2], cudaStreamNonBlocking));
+  }
+  while (true) {
+    int rc = I.tuned ? BES_OK : tune_sweep<T, B>(c);
+    if (rc) return rc;
+    rc = make_step_graph<T, B>(c, prof);
+    if (rc == BES_OK || (I.solve_blocks == 0 && I.sweep_kernel != 2)) return rc;
+    drop_persistent(c, "could not be captured in the step graph");
+  }
 }
 
 // ---- host side of a step -------------------------------------------------------------------
@@ -950,7 +979,15 @@ int run_steps(bes_ctx* c, int64_t n, double* history) {
   for (int64_t i = 0; i < n; ++i) {
     int rc = upload_step_inputs(c, act, cfl, P);
     if (rc) return rc;
-    IMP_TRY(c, cudaGraphLaunch(I.step_graph[prof][c->cur], c->stream));
+    if (cudaGraphLaunch(I.step_graph[prof][c->cur], c->stream) != cudaSuccess &&
+        (I.solve_blocks > 0 || I.sweep_kernel == 2)) {
+      // refused at its launch
+      cudaGetLastError();
+      IMP_TRY(c, cudaStreamSynchronize(c->stream));
+      drop_persistent(c, "was refused");
+      if ((rc = build_step_graph<T, B>(c, prof))) return rc;
+      IMP_TRY(c, cudaGraphLaunch(I.step_graph[prof][c->cur], c->stream));
+    }
     int nan = 0, sync_err = 0;
     unsigned long long cnt[3];
     IMP_TRY(c, cudaMemcpyAsync(I.res_host.data(), I.res, ns * sizeof(StepResult),
@@ -964,7 +1001,10 @@ int run_steps(bes_ctx* c, int64_t n, double* history) {
     if (sync_err) {
       if ((rc = reset_grid_sync(c))) return rc;
       check_step_nan(c, nan);  // the flag is the failed step's
-      c->last_error = "a wait of the linear solves gave up after one second; the step was not applied";
+      const bool solve = I.solve_blocks > 0;
+      drop_persistent(c, "gave up waiting");
+      c->last_error = std::string("a wait of the persistent ") + (solve ? "linear solve" : "colour sweep") +
+                      " gave up after one second; the step was not applied, and the next ones run without it";
       return BES_ERR_TIMEOUT;
     }
     // kernels this step launched: the graph's top level, the assembly of each slot that
@@ -1296,8 +1336,12 @@ int bes_set_linear_guard(bes_ctx* ctx, int32_t max_cycles) {
 }
 
 int bes_inject_failure(bes_ctx* ctx, int32_t what) {
-  if (!ctx || what != BES_FAIL_WAIT) return BES_ERR_INVALID;
+  if (!ctx || what < BES_FAIL_WAIT || what > BES_FAIL_SOLVE_CAPTURE) return BES_ERR_INVALID;
   if (ctx->opt.solver_type != 1 || !ctx->imp.sync_error) return BES_ERR_INVALID;
+  if (what != BES_FAIL_WAIT) {
+    ctx->imp.inject = what;
+    return BES_OK;
+  }
   const int on = 1;
   IMP_TRY(ctx, cudaMemcpyAsync(ctx->imp.sync_error, &on, sizeof(int), cudaMemcpyHostToDevice, ctx->stream));
   IMP_TRY(ctx, cudaStreamSynchronize(ctx->stream));

@@ -163,7 +163,7 @@ int bes_explicit_iterations(bes_ctx* ctx, int64_t n, double* history);
  * step; its history rows are zeros.  Returns BES_ERR_TIMEOUT when a linear solve was stopped
  * by its restart-cycle limit (bes_set_linear_guard), with the step applied, or when a wait
  * between the blocks of a persistent kernel gave up, with the state as it was before the step; the
- * context stays usable. */
+ * context stays usable and does not take that kernel again. */
 int bes_implicit_steps(bes_ctx* ctx, int64_t n, double* history);
 
 /* Implicit-path statistics: out[0] steps taken, out[1] host synchronisations inside
@@ -183,8 +183,11 @@ int bes_set_linear_guard(bes_ctx* ctx, int32_t max_cycles);
 
 /* Test aid: a failure made on the host, for the context's next implicit step.
  *   BES_FAIL_WAIT  the flag that a wait of the linear solves sets when it gives up is set before
- *                  the step: the step is not applied and returns BES_ERR_TIMEOUT. */
+ *                  the step: the step is not applied and returns BES_ERR_TIMEOUT.
+ *   BES_FAIL_SOLVE_CAPTURE  (before the first step) the one-launch linear solve is refused when the
+ *                  step graph is made: the step runs with the graph's own solve. */
 #define BES_FAIL_WAIT 1
+#define BES_FAIL_SOLVE_CAPTURE 2
 int bes_inject_failure(bes_ctx* ctx, int32_t what);
 
 /* Assemble (without solving or updating) the implicit system at the current state and CFL

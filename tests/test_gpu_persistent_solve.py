@@ -55,3 +55,34 @@ def test_step_whose_wait_gave_up_is_not_applied(precision, sweep_kernel, n_cond)
     assert np.array_equal(c.implicit_steps(1), h2)
     assert np.array_equal(c.get_state(), U2)
     c.close()
+
+
+def _three_steps(failure, at, precision, linear, profile=False):
+    """Three steps with a failure injected before step `at`; histories, state and the tuning text."""
+    c = context(meshgen.bump_channel(9, 3, 1, 0.08), precision=precision, linear_solver=linear, **OPTS)
+    c.profile(profile)
+    h = []
+    for k in range(3):
+        if k == at:
+            c.inject_failure(failure)
+        try:
+            h.append(c.implicit_steps(1))
+        except lib.BesError as e:
+            assert e.code == 7 and failure == lib.FAIL_WAIT and k == at
+            h.append(c.implicit_steps(1))
+    U, text = c.get_state(), c.tuning()
+    c.close()
+    return np.concatenate(h), U, text
+
+
+@pytest.mark.parametrize("failure,at", [(lib.FAIL_SOLVE_CAPTURE, 0), (lib.FAIL_WAIT, 1)])
+@pytest.mark.parametrize("precision", [0, 1, 2])
+@pytest.mark.parametrize("linear", [0, 1])
+def test_refused_solve_falls_back_to_the_graph(failure, at, precision, linear):
+    """Refused when the step graph is made, or given up in a step: the steps are those of a
+    context in which nothing failed, and the persistent form is not taken again."""
+    h, U, text = _three_steps(0, -1, precision, linear)
+    assert "taken: the step graph's solve" not in text
+    hf, Uf, textf = _three_steps(failure, at, precision, linear, profile=failure == lib.FAIL_WAIT)
+    assert textf.count("taken: the step graph's solve") == 1
+    assert np.array_equal(hf, h) and np.array_equal(Uf, U)
