@@ -644,7 +644,16 @@ void choose_solve(bes_ctx* c) {
   const double held = (double)kRowsPerWarp * 8 * blocks;
   if (stage > held * (uses_ilu(c) ? 1.6 : 5.5)) return;
   I.solve_lane_spmv = rows <= 1.25 * held;
-  if (uses_ilu(c) && !I.Y && imp_malloc(c, &I.Y, I.ldv * I.tsize * I.nslot)) return;
+  if (uses_ilu(c) && !I.Y) {
+    // (2^60 bytes: more than any device gives)
+    const size_t bytes = I.inject == BES_FAIL_SOLVE_ALLOC ? (size_t)1 << 60 : I.ldv * I.tsize * I.nslot;
+    I.inject = I.inject == BES_FAIL_SOLVE_ALLOC ? 0 : I.inject;
+    if (imp_malloc(c, &I.Y, bytes)) {
+      cudaGetLastError();  // the step does without it
+      I.Y = nullptr;
+      return;
+    }
+  }
   I.solve_blocks = (int)blocks;
 }
 
@@ -1336,7 +1345,7 @@ int bes_set_linear_guard(bes_ctx* ctx, int32_t max_cycles) {
 }
 
 int bes_inject_failure(bes_ctx* ctx, int32_t what) {
-  if (!ctx || what < BES_FAIL_WAIT || what > BES_FAIL_SOLVE_CAPTURE) return BES_ERR_INVALID;
+  if (!ctx || what < BES_FAIL_WAIT || what > BES_FAIL_SOLVE_ALLOC) return BES_ERR_INVALID;
   if (ctx->opt.solver_type != 1 || !ctx->imp.sync_error) return BES_ERR_INVALID;
   if (what != BES_FAIL_WAIT) {
     ctx->imp.inject = what;

@@ -38,7 +38,7 @@ EXPORTED = [
 ]
 
 OUTPUT_VTK, OUTPUT_CSV, OUTPUT_SLIP_WALL_CSV = 0, 1, 2
-FAIL_WAIT, FAIL_SOLVE_CAPTURE = 1, 2
+FAIL_WAIT, FAIL_SOLVE_CAPTURE, FAIL_SOLVE_ALLOC = 1, 2, 3
 
 
 class BesError(RuntimeError):

@@ -185,9 +185,11 @@ int bes_set_linear_guard(bes_ctx* ctx, int32_t max_cycles);
  *   BES_FAIL_WAIT  the flag that a wait of the linear solves sets when it gives up is set before
  *                  the step: the step is not applied and returns BES_ERR_TIMEOUT.
  *   BES_FAIL_SOLVE_CAPTURE  (before the first step) the one-launch linear solve is refused when the
- *                  step graph is made: the step runs with the graph's own solve. */
+ *                  step graph is made: the step runs with the graph's own solve.
+ *   BES_FAIL_SOLVE_ALLOC  (before the first step) its vector cannot be allocated: the same. */
 #define BES_FAIL_WAIT 1
 #define BES_FAIL_SOLVE_CAPTURE 2
+#define BES_FAIL_SOLVE_ALLOC 3
 int bes_inject_failure(bes_ctx* ctx, int32_t what);
 
 /* Assemble (without solving or updating) the implicit system at the current state and CFL

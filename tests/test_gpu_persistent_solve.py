@@ -86,3 +86,13 @@ def test_refused_solve_falls_back_to_the_graph(failure, at, precision, linear):
     hf, Uf, textf = _three_steps(failure, at, precision, linear, profile=failure == lib.FAIL_WAIT)
     assert textf.count("taken: the step graph's solve") == 1
     assert np.array_equal(hf, h) and np.array_equal(Uf, U)
+
+
+@pytest.mark.parametrize("precision", [0, 1, 2])
+def test_no_memory_for_the_solve(precision):
+    """The graph's solve, with every colour-sweep form in the running (the allocation's error, left
+    for the next check, took the first form out of it)."""
+    h, U, _ = _three_steps(0, -1, precision, 1)
+    hf, Uf, text = _three_steps(lib.FAIL_SOLVE_ALLOC, 0, precision, 1)
+    assert "one persistent launch" not in text and "one launch per colour failed" not in text
+    assert np.array_equal(hf, h) and np.array_equal(Uf, U)
