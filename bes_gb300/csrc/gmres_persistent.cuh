@@ -2,13 +2,13 @@
 // preconditioner sweep and GMRES decision of all slots.
 //
 // On meshes whose phases take a few microseconds the step graph's solve is bound by its nodes:
-// an Arnoldi step is 14 kernels and two conditional nodes, about 100 us from 1,152 to 75,000
-// cells whatever the precision.  Here nothing is launched between Arnoldi steps: rows wait for
+// an Arnoldi step with block ILU is 12 kernels (eight of them the colour sweep's) and two conditional
+// nodes: 57 to 80 us from 1,152 to 50,000 cells in FP32, 95 to 139 in FP64.  Here nothing is launched between Arnoldi steps: rows wait for
 // the entries they need (below), four grid barriers (an atomic and a poll of one word in L2, about
 // 2 us) separate the product, the dot products, their reduction and the new basis vector, and
 // the decisions are taken by every block from the same values.  What is left is a chain of
-// round trips to L2: about 45 us an Arnoldi step at 7,000 to 20,000 cells (sweeps 22, product
-// 5, Gram-Schmidt 17).
+// round trips to L2: an Arnoldi step takes 41 to 50 us in FP32 (7,000 cells: sweeps 20, product
+// 5, Gram-Schmidt 17), 48 to 50 in FP64 up to 7,000 cells and 85 at 31,000.
 //
 // Every value is computed as by the graph's kernels, bit for bit: rows in the order of the row
 // functions, reductions over the same kRedBlocks x 256 threads ("virtual blocks", dealt out to

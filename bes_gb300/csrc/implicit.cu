@@ -621,12 +621,27 @@ int reset_grid_sync(bes_ctx* c) {
 }
 
 // The linear solves as one persistent launch (gmres_persistent.cuh) or as the graph's kernels:
-// persistent while the rows between two waits (a colour, or all of them with block Jacobi) are
-// no more than a few times what the grid's warps hold at six rows each.  Two steps at CFL 50, graph
-// against persistent, measured in ms with the multiple in brackets: block ILU FP32 12k cells 7.5 /
-// 5.0, 52k 12.1 / 7.4, 74k (1.0) 13.7 / 12.5, 130k (1.8) 19.2 / 19.8; FP64 12k 13.3 / 7.0, 52k (1.4)
-// 21.5 / 20.2, 74k (2.0) 25.9 / 27.9; packed 12k 7.8 / 5.3, 74k (1.0) 13.5 / 10.9.  Block Jacobi: FP64
-// 33k (4.5) 29.3 / 22.5, FP32 74k (5.1) 21.1 / 16.2.
+// persistent while the rows between two waits (a colour, or all of them with block Jacobi) are no
+// more than a multiple of what the grid's warps hold at six rows each.  The grid has one block an
+// SM in FP64 and two otherwise, and a stage that needs one more turn of the grid than another
+// takes longer by a step, so the line lies elsewhere for each storage.  Two steps at CFL 50, ms,
+// graph / persistent, the multiple in brackets:
+//   block ILU  FP64    7k 9.2 / 5.1   40k (1.1) 17.3 / 15.1   46k (1.25) 19.0 / 17.1   51k (1.4) 19.3 / 19.9
+//              FP32    7k 5.5 / 4.0   72k (0.98) 12.7 / 10.4   74k (1.02) 12.4 / 12.2   83k (1.14) 13.9 / 15.1
+//              16-bit  7k 5.6 / 4.3   91k (1.25) 14.4 / 13.7   110k (1.5) 15.6 / 15.5   121k (1.65) 15.7 / 16.5
+//   Jacobi     FP64    7k 11.7 / 6.7   40k (5.4) 26.8 / 25.1   45k (6.1) 28.5 / 27.6   50k (6.8) 29.4 / 32.5
+//              FP32    7k 8.0 / 5.9   70k (4.8) 17.2 / 16.6   74k (5.1) 16.8 / 15.7   83k (5.7) 18.7 / 20.0
+//              16-bit  7k 7.8 / 6.2   101k (6.9) 18.0 / 17.6   110k (7.5) 19.0 / 18.3   130k (8.9) 20.6 / 24.2
+// Conditions count as rows: four of 20k in FP32 (1.11) 10.8 / 10.4, thirty of 1k in FP64 38.8 / 23.6.
+// Its products take one component per lane where the rows leave lanes idle otherwise: FP64 block
+// ILU / Jacobi, rows against lanes, 4k 5.24 / 4.97 and 6.62 / 6.01, 7k (rows 0.95 of what is held)
+// 5.28 / 5.05 and 7.31 / 6.69, 10k (1.35) 5.81 / 5.85 and 8.88 / 8.73, 15k 6.82 / 7.04 and 9.71 /
+// 10.44; FP32 and 16-bit block ILU never (4k 3.81 / 3.86, 15k 4.96 / 5.27), block Jacobi 4k 5.37 /
+// 5.31 and 5.80 / 5.63, 11k (0.75) 7.12 / 7.15 and 7.75 / 7.58, 15k (1.0) 7.49 / 8.38 and 8.09 / 8.70.
+// The launch takes every SM: contexts stepped at the same time from several threads take turns,
+// where the graph's kernels overlap (sweep_kernel = 1).  ms a step of all, 7k FP64 block Jacobi, 1 /
+// 2 / 3 / 4 contexts: 2.7 / 5.3 / 8.0 / 10.7, graph 4.7 / 6.1 / 7.7 / 9.1; 50k 16-bit block ILU 3.4 /
+// 6.6 / 9.8 / 13.0, graph 4.9 / 5.7 / 6.2 / 6.7.
 void choose_solve(bes_ctx* c) {
   ImplicitBuffers& I = c->imp;
   I.solve_blocks = 0;
@@ -642,8 +657,10 @@ void choose_solve(bes_ctx* c) {
   }
   const int64_t blocks = std::min<int64_t>(I.solve_resident, (rows + 31) / 32);
   const double held = (double)kRowsPerWarp * 8 * blocks;
-  if (stage > held * (uses_ilu(c) ? 1.6 : 5.5)) return;
-  I.solve_lane_spmv = rows <= 1.25 * held;
+  const bool ilu = uses_ilu(c);
+  const double limit = !I.prec ? (ilu ? 1.3 : 6.2) : I.packed ? (ilu ? 1.5 : 7.5) : (ilu ? 1.05 : 5.3);
+  if (stage > held * limit) return;
+  I.solve_lane_spmv = rows <= held * (!I.prec ? 1.25 : ilu ? 0.0 : 0.8);
   if (uses_ilu(c) && !I.Y) {
     // (2^60 bytes: more than any device gives)
     const size_t bytes = I.inject == BES_FAIL_SOLVE_ALLOC ? (size_t)1 << 60 : I.ldv * I.tsize * I.nslot;

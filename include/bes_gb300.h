@@ -93,7 +93,10 @@ typedef struct {
                                      0 the autotuner's choice (timed on the first step's
                                      system, see bes_tuning), 1 one launch per colour, 2 one
                                      persistent launch per sweep, 3 one launch per colour
-                                     with every load of a row issued first (precision 2) */
+                                     with every load of a row issued first (precision 2).
+                                     0 also lets the linear solves of a small system run as one
+                                     launch, which takes the whole GPU: 1 is the faster choice
+                                     where several contexts are stepped at the same time */
   int32_t reserved_i;
   double reserved[2];
 } bes_options;
