@@ -770,7 +770,7 @@ struct bes_mlp {
   int device = 0;
   cudaStream_t stream = nullptr;
   std::string last_error;
-  std::vector<void*> allocs;
+  std::vector<void*> allocs, batch_allocs;
   int64_t nc = 0, n_rows = 0;  // cells, cells rounded up to the row tile
   double gamma = 1.4, R = 287.0;
   Layout L;
@@ -821,41 +821,58 @@ int gemm_status(bes_mlp* h) {
 }
 
 template <class X>
-int mlp_alloc(bes_mlp* h, X** ptr, size_t count) {
+int mlp_alloc(bes_mlp* h, X** ptr, size_t count, std::vector<void*>& list) {
   *ptr = nullptr;
   cudaError_t e = cudaMalloc((void**)ptr, std::max<size_t>(count, 1) * sizeof(X));
   if (e != cudaSuccess) {
+    cudaGetLastError();  // not the next call's
     h->last_error = std::string("cudaMalloc: ") + cudaGetErrorString(e);
     return BES_ERR_CUDA;
   }
-  h->allocs.push_back(*ptr);
+  list.push_back(*ptr);
   return BES_OK;
 }
+template <class X>
+int mlp_alloc(bes_mlp* h, X** ptr, size_t count) {
+  return mlp_alloc(h, ptr, count, h->allocs);
+}
 
+void free_batch(bes_mlp* h) {
+  for (void* q : h->batch_allocs) cudaFree(q);
+  h->batch_allocs.clear();
+  h->cap = 0;
+}
+
+// Buffers for batches of B rows: all of them or none, in place of smaller ones.
 int ensure_batch(bes_mlp* h, int B) {
   if (B <= h->cap) return BES_OK;
+  free_batch(h);
   int rc = 0;
-  rc |= mlp_alloc(h, &h->H0, (size_t)B * kK0);
-  rc |= mlp_alloc(h, &h->H0T, (size_t)B * kK0);
+  auto alloc = [&](auto** ptr, size_t count) { rc |= mlp_alloc(h, ptr, count, h->batch_allocs); };
+  alloc(&h->H0, (size_t)B * kK0);
+  alloc(&h->H0T, (size_t)B * kK0);
   const int chunks = B / kChunk;
   for (int l = 0; l < kLayers; ++l) {
-    rc |= mlp_alloc(h, &h->ZT[l], (size_t)B * kW);
-    rc |= mlp_alloc(h, &h->HT[l], (size_t)B * kW);
-    rc |= mlp_alloc(h, &h->dZT[l], (size_t)B * kW);
-    rc |= mlp_alloc(h, &h->part[l], (size_t)chunks * 9 * kW);
+    alloc(&h->ZT[l], (size_t)B * kW);
+    alloc(&h->HT[l], (size_t)B * kW);
+    alloc(&h->dZT[l], (size_t)B * kW);
+    alloc(&h->part[l], (size_t)chunks * 9 * kW);
     // split-K partials of dW: B / 512 splits of [256][K]
-    rc |= mlp_alloc(h, &h->wpart[l], (size_t)std::max(1, B / 512) * kW * (l == 0 ? kK0 : kW));
+    alloc(&h->wpart[l], (size_t)std::max(1, B / 512) * kW * (l == 0 ? kK0 : kW));
   }
-  rc |= mlp_alloc(h, &h->C, (size_t)B * 3);
-  rc |= mlp_alloc(h, &h->T, (size_t)B * kOut);
-  rc |= mlp_alloc(h, &h->O, (size_t)B * 8);
-  rc |= mlp_alloc(h, &h->dO, (size_t)B * 8);
-  rc |= mlp_alloc(h, &h->dHT, (size_t)B * kW);
-  rc |= mlp_alloc(h, &h->dZ, (size_t)B * kW);
-  rc |= mlp_alloc(h, &h->part4, (size_t)chunks * (kOut * kW + kOut));
-  rc |= mlp_alloc(h, &h->row_loss, (size_t)B);
-  rc |= mlp_alloc(h, &h->loss_part, (size_t)(B + 255) / 256);
-  if (rc) return BES_ERR_CUDA;
+  alloc(&h->C, (size_t)B * 3);
+  alloc(&h->T, (size_t)B * kOut);
+  alloc(&h->O, (size_t)B * 8);
+  alloc(&h->dO, (size_t)B * 8);
+  alloc(&h->dHT, (size_t)B * kW);
+  alloc(&h->dZ, (size_t)B * kW);
+  alloc(&h->part4, (size_t)chunks * (kOut * kW + kOut));
+  alloc(&h->row_loss, (size_t)B);
+  alloc(&h->loss_part, (size_t)(B + 255) / 256);
+  if (rc) {
+    free_batch(h);
+    return BES_ERR_CUDA;
+  }
   h->cap = B;
   return BES_OK;
 }
@@ -1107,6 +1124,7 @@ void bes_mlp_destroy(bes_mlp* h) {
   if (!h) return;
   for (cudaStream_t s : {h->stream, h->copy})
     if (s) cudaStreamSynchronize(s);
+  free_batch(h);
   for (void* q : h->allocs) cudaFree(q);
   for (int b = 0; b < 2; ++b) {
     if (h->ready[b]) cudaEventDestroy(h->ready[b]);
