@@ -805,7 +805,8 @@ __global__ void __launch_bounds__(256, std::is_same<T, double>::value ? 1 : 2) g
   __shared__ int second_sh[kMaxSlots];
   __shared__ int run_sh[kMaxSlots];  // the flags of the current phases
   // the arguments in shared memory: the phases are functions of their own (inlined into one body
-  // they spill, and a spilled register comes back from L2 behind every barrier)
+  // they spill 500 to 1400 bytes, and a spilled register comes back from L2 behind every barrier;
+  // as functions 68 bytes in FP32 and none in FP64)
   __shared__ __align__(16) unsigned char args_sh[sizeof(SolveArgs<T, B>)];
   for (unsigned q = threadIdx.x; q < sizeof(SolveArgs<T, B>) / 4; q += 256)
     reinterpret_cast<unsigned*>(args_sh)[q] = reinterpret_cast<const unsigned*>(&args)[q];

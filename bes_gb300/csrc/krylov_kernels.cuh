@@ -290,7 +290,7 @@ __global__ void __launch_bounds__(128, 12) ilu_colour_packed_kernel(
 // (neighbour ids, then everything else) instead of one per qualifying slot, at the cost of
 // registers.  The arithmetic is that of ilu_colour_packed_row in the same order, so the
 // results are identical; the autotuner keeps it only where it is faster.
-template <bool LOWER, bool UPPER, bool COH = false>
+template <bool LOWER, bool UPPER>
 __device__ __forceinline__ void ilu_colour_packed_row_ld(
     const DevMesh& m, int i, int r0, int r1, int s1, const uint32_t* __restrict__ H,
     const uint32_t* __restrict__ D, const float* __restrict__ in, float* __restrict__ out) {
@@ -301,7 +301,7 @@ __device__ __forceinline__ void ilu_colour_packed_row_ld(
 #pragma unroll
   for (int s = 0; s < 4; ++s) jn[s] = m.adj[s * nc + i];
   float acc[5];
-  gather5<COH>(own, i, acc);
+  gather5(own, i, acc);
   bool q[4];
   PackedBlock blk[4];
   float y[4][5];
@@ -314,7 +314,7 @@ __device__ __forceinline__ void ilu_colour_packed_row_ld(
     if (q[s]) {
       const float* src = (lower && j < s1) ? in : out;
       blk[s] = load_packed_once(H, 4, s, i, pol);
-      gather5<COH>(src, j, y[s]);
+      gather5(src, j, y[s]);
     }
   }
 #pragma unroll
@@ -357,7 +357,7 @@ __global__ void __launch_bounds__(128) ilu_colour_packed_ld_kernel(
 
 // ---- persistent colour sweep ----------------------------------------------------------------
 // One launch per preconditioner application: a grid of resident blocks (cooperative launch,
-// sized by occupancy) walks the 2C-1 colour stages of the sweep in order, the rows of every
+// sized by occupancy) walks the 2C-2 colour stages of the sweep in order, the rows of every
 // slot of a stage spread over all its threads, with a grid barrier between stages.  Each row
 // computes exactly what the per-colour kernels compute.  Vector values written in one stage
 // are read in later stages by other blocks, so those loads go through L2 (vld<true>).
@@ -564,11 +564,11 @@ __global__ void __launch_bounds__(256) copy_vec_kernel(SlotPtr<T> outp, SlotPtr<
 }
 
 // block-Jacobi application: out_i = Dinv_i in_i
-template <class T, bool COH>
+template <class T>
 __device__ __forceinline__ void jacobi_row(int i, const T* __restrict__ Dinv, const T* in, T* out) {
   T x[5], a[25];
   load_block_once(Dinv, 1, 0, i, a, l2_evict_first());
-  gather5<COH>(in, i, x);
+  gather5(in, i, x);
 #pragma unroll
   for (int r = 0; r < 5; ++r) {
     T acc = T(0);
@@ -583,16 +583,15 @@ __global__ void __launch_bounds__(256) jacobi_apply_kernel(int nc, SlotPtr<const
                                                            const int32_t* run) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= nc || slot_idle(run)) return;
-  jacobi_row<T, false>(i, Dp.at(), inp.at(), outp.at());
+  jacobi_row<T>(i, Dp.at(), inp.at(), outp.at());
 }
 
 // block-Jacobi application with a packed inverse diagonal
-template <bool COH>
 __device__ __forceinline__ void jacobi_packed_row(int i, const uint32_t* __restrict__ D, const float* in,
                                                   float* out) {
   float x[5], a[25];
   const PackedBlock blk = load_packed(D, 1, 0, i);
-  gather5<COH>(in, i, x);
+  gather5(in, i, x);
   const float sc = blk.unpack(a);
 #pragma unroll
   for (int r = 0; r < 5; ++r) {
@@ -607,7 +606,7 @@ static __global__ void __launch_bounds__(256) jacobi_apply_packed_kernel(
     const int32_t* run) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= nc || slot_idle(run)) return;
-  jacobi_packed_row<false>(i, Dp.at(), inp.at(), outp.at());
+  jacobi_packed_row(i, Dp.at(), inp.at(), outp.at());
 }
 
 // ---- matrix-vector products ------------------------------------------------------------------
@@ -1169,8 +1168,9 @@ enum GsMode { GS_FINAL1 = 0, GS_REORTH = 1, GS_FINAL2 = 2 };
 // a second pass) or h2 (FINAL2, runs with one); with an FP16 basis the new vector also goes to
 // outx in T (the preconditioner's input).  REORTH: w -= sum_k h_k V_k in place, with partial
 // V_k . w (rows k < NV) and |w|^2 (row NV) of the result.
-// (the registers of the Givens block must not cost the other blocks their residency: with an FP16
-// basis they need 34 to 44)
+// (the registers of the Givens block must not cost the other blocks their residency: six of them need
+// 40 registers a thread, with which the loop alone spills 12 bytes at most, and 20 to 108 beside
+// the Givens block)
 template <class B, int MODE>
 constexpr int kGsBlocks = sizeof(B) == 2 && MODE != GS_REORTH ? 6 : 1;
 template <class T, class B, int NV, int MODE>

@@ -21,10 +21,10 @@
 //     (Halley for 1/x, Householder for 1/sqrt(x)): at most 1 and 2 ulp measured over 2^-60..2^60.
 // FP64 instructions per cell and stage (Nf/Nc = 2): about 570 + 420 + 30 before, 180 + 155 + 27.
 //
-// Implicit steps keep the kernels of explicit_kernels.cuh: the linear solves of the FP32 and
-// 16-bit systems amplify a rounding difference of the right-hand side (1e-15 becomes 5e-9 and
-// 5e-7 of the state after one step), and the three precisions start from one residual, bit for
-// bit.  A step spends 1 to 6 % of its time there.
+// Implicit steps keep the kernels of explicit_kernels.cuh, and with them the bits of their results:
+// the linear solves of the FP32 and 16-bit systems amplify a rounding difference of the right-hand
+// side (1e-15 becomes 5e-9 and 5e-7 of the state after one step, well inside the solves' own
+// tolerance).  The residual is 7 to 8 % of a step on 2.16M cells in 16-bit storage.
 #pragma once
 #include "explicit_kernels.cuh"
 
