@@ -60,9 +60,13 @@ __device__ __forceinline__ double fast_rsqrt(double x) {
   const double e = fma(-x * y, y, 1.0);
   return fma(y * e, fma(e, 0.375, 0.5), y);
 }
-// sqrt(x) by the same; sqrt(0) is 0 (0 * 1/sqrt(0) is a NaN: a cell without pressure is a valid state)
-__device__ __forceinline__ double fast_sqrt(double x) {
-  return mid_range(x) ? x * fast_rsqrt(x) : sqrt(x);
+// sqrt(x) as a product s y, so that adding to it is one fma: x times 1/sqrt(x), or sqrt(x) times 1
+// outside of the range (0 times 1/sqrt(0) is a NaN, and a cell without pressure is a valid state)
+struct RootFactors {
+  double s, y;
+};
+__device__ __forceinline__ RootFactors fast_sqrt(double x) {
+  return mid_range(x) ? RootFactors{x, fast_rsqrt(x)} : RootFactors{sqrt(x), 1.0};
 }
 __device__ __forceinline__ long long dbits(double x) { return __double_as_longlong(x); }
 // a <= b for a, b >= 0 (or a NaN, which compares greater than every number)
@@ -142,10 +146,11 @@ __device__ __forceinline__ double local_time_step(const DevMesh& m, const Params
   for (int d = 0; d < 3; ++d) w[d] = u[1 + d] * ir;
   const double k = fma(u[1], w[0], fma(u[2], w[1], u[3] * w[2]));
   const double cs2 = g.gamma2_gm1 * fma(-0.5, k, u[4]) * ir;
-  const double cs = fast_sqrt(cs2);
+  const RootFactors cs = fast_sqrt(cs2);
   double spec = 0.0;
 #pragma unroll
-  for (int d = 0; d < 3; ++d) spec = fma(cs + fabs(w[d]), m.plen[(int64_t)d * m.nc + c], spec);
+  for (int d = 0; d < 3; ++d)
+    spec = fma(fma(cs.s, cs.y, fabs(w[d])), m.plen[(int64_t)d * m.nc + c], spec);
   return cfl * m.vol[c] * fast_rcp(spec);
 }
 

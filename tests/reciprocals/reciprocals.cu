@@ -6,7 +6,8 @@ __global__ void reciprocals_kernel(const double* x, int64_t n, double* out) {
   if (i >= n) return;
   out[i] = bes::fast_rcp(x[i]);
   out[n + i] = bes::fast_rsqrt(x[i]);
-  out[2 * n + i] = bes::fast_sqrt(x[i]);
+  const bes::RootFactors r = bes::fast_sqrt(x[i]);
+  out[2 * n + i] = r.s * r.y;
 }
 
 extern "C" int reciprocals(const double* x, int64_t n, double* out) {
